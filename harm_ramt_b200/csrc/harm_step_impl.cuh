@@ -4,6 +4,7 @@
 // built with contraction and fast FP32 division/square root).
 #pragma once
 #include <cuda_runtime.h>
+#include "harm_exact.cuh"
 #include "harm_kernels.cuh"
 #include "harm_tma.cuh"
 
@@ -32,6 +33,56 @@ __device__ __forceinline__ void zone_states(const double* t, int ps, int st, T* 
       para4((T)pk[-2 * st], (T)pk[-st], (T)pk[0], (T)pk[st], (T)pk[2 * st], l, r);
       L[k] = l;
       R[k] = r;
+    }
+  }
+}
+
+// The FP64 interface states of N consecutive zones of one variable, a thread
+// walking along the zones (src: the first zone's value, step st; one more
+// value on each side is read for MC, two for PARA).  The slopes and, for
+// PARA, the raw interface values that neighbouring zones share are formed
+// once; put(c, l, r) takes zone c's states.  The values are mc_slope's and
+// para4's: 2 min(|a|, |b|) is min(|2 a|, |2 b|), (4 a) b is (2 a)(2 b), and
+// the sign of a slope is copied instead of multiplied.
+__device__ __forceinline__ double para_dq_shared(double a, double b, double ym, double yp)
+{
+  const double s = (4. * a) * b, c = 0.5 * (yp - ym);
+  const double m = 2. * rmin(fabs(a), fabs(b));
+  return (s <= 0.) ? 0. : copysign(rmin(fabs(c), m), c);
+}
+template <bool PARA, int N, typename Put>
+__device__ __forceinline__ void row_states(const double* src, int st, Put put)
+{
+  double ym = src[-st], y = src[0], a = y - ym;
+  if (!PARA) {
+#pragma unroll
+    for (int c = 0; c < N; c++) {
+      const double yp = src[(c + 1) * st], b = yp - y;
+      const double h = 0.5 * minmod(0.5 * (yp - ym), minmod(2. * a, 2. * b));
+      put(c, y - h, y + h);
+      ym = y;
+      y = yp;
+      a = b;
+    }
+  } else {
+    double yp = src[st], b = yp - y;
+    const double ymm = src[-2 * st];
+    double d0 = para_dq_shared(ym - ymm, a, ymm, y), d = para_dq_shared(a, b, ym, yp);
+    double l = para_face(ym, y, d0, d);
+#pragma unroll
+    for (int c = 0; c < N; c++) {
+      const double ypp = src[(c + 2) * st], e = ypp - yp;
+      const double d1 = para_dq_shared(b, e, y, ypp);
+      const double r = para_face(y, yp, d, d1);
+      double lo, ro;
+      para_limit(ym, y, yp, l, r, lo, ro);
+      put(c, lo, ro);
+      ym = y;
+      y = yp;
+      yp = ypp;
+      b = e;
+      d = d1;
+      l = r;
     }
   }
 }
@@ -104,6 +155,237 @@ __device__ __forceinline__ void face_flux(const StepArgs& a, int i, int j, int d
   dtij = a.pp.cour * (dir == 1 ? a.pp.dx1 : a.pp.dx2) / cm;
 }
 
+// ---- the FP64 face without branches (harm_exact.cuh)
+// The functions below evaluate get_state, primtoflux, vchar and the Riemann
+// flux (the templates of harm_device.cuh and face_flux above) with the same
+// operands in the same order, every quotient and root through `ex`.  While
+// ex.ok() holds every value is finite and in range, so sums leave out the
+// terms that are a value times an exact zero or an exact zero itself (the
+// unit covectors of vchar, the Kronecker delta of mhd_calc_0, the B^dir row).
+// Where the templates branch (a Lorentz limit, a wavespeed outside its
+// bounds) ex.ok() is false and the face goes through face_flux.
+
+// lapse and shift of a location, as ucon_calc_rel4vel forms them
+struct LapseX {
+  Recip alpha;
+  double beta[3];
+};
+__device__ __forceinline__ LapseX lapse_x(Exact& ex, const double* gcon)
+{
+  LapseX l;
+  const double alpha = Exact::quot(1., ex.rcp(ex.sqrt_of(-gcon[0])));
+  l.alpha = ex.rcp(alpha);
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    l.beta[k] = gcon[1 + k] * alpha * alpha;
+    ex.numerator<-600>(l.beta[k]);
+  }
+  return l;
+}
+
+struct StateX : State<double> {
+  Recip ut;  // u^t
+  double bsq, gamma;
+};
+// get_state; limit: GAMMAMAX where the caller limits the Lorentz factor first
+template <typename EX>
+__device__ __forceinline__ void state_x(EX& ex, const double* pr, const double* c, const LapseX& l, double limit,
+                                        StateX& q)
+{
+  const double qsq = c[4] * pr[U1] * pr[U1] + c[7] * pr[U2] * pr[U2] + c[9] * pr[U3] * pr[U3] +
+                     2. * (c[5] * pr[U1] * pr[U2] + c[6] * pr[U1] * pr[U3] + c[8] * pr[U2] * pr[U3]);
+  const double gamma = ex.sqrt_of(1. + qsq);
+  ex.need(gamma <= limit);
+  q.gamma = gamma;
+  q.ucon[0] = Exact::quot(gamma, l.alpha);
+#pragma unroll
+  for (int k = 0; k < 3; k++) q.ucon[1 + k] = pr[U1 + k] - Exact::quot(gamma * l.beta[k], l.alpha);
+  lower_v(q.ucon, c, q.ucov);
+  q.bcon[0] = pr[B1] * q.ucov[1] + pr[B2] * q.ucov[2] + pr[B3] * q.ucov[3];
+  q.ut = ex.rcp(q.ucon[0]);
+#pragma unroll
+  for (int k = 1; k < 4; k++) q.bcon[k] = ex.div(pr[B1 - 1 + k] + q.bcon[0] * q.ucon[k], q.ut);
+  lower_v(q.bcon, c, q.bcov);
+  q.bsq = dot4(q.bcon, q.bcov);
+}
+
+// What a face takes from one interface state.  The B^dir row of the flux and
+// of the conserved vectors' difference is zero on both sides (B^dir is
+// continuous), so two field components are kept: the other one of the plane
+// and B3.
+constexpr int NX = NPR - 1, XB = B1, XB3 = B1 + 1;
+struct SideX {
+  double F[NX], U[NX], vmax, vmin;
+};
+
+// primtoflux in direction dir (1 or 2) and in time, and vchar; sg: sqrt(-g);
+// gd, gdd: g^{t dir} and g^{dir dir}
+template <bool FFDE, typename EX>
+__device__ __forceinline__ void side_x(EX& ex, const double* pr, const StateX& q, int dir, double sg, double gtt,
+                                       double gd, double gdd, double gam, SideX& x)
+{
+  const bool d1 = (dir == 1);
+  {
+    const double r = FFDE ? 0. : pr[RHO], u = FFDE ? 0. : pr[UU], P = (gam - 1.) * u, w = P + r + u;
+    const double eta = FFDE ? q.bsq : w + q.bsq, ptot = FFDE ? q.bsq * 0.5 : P + q.bsq * 0.5;
+    const double ud = d1 ? q.ucon[1] : q.ucon[2], bd = d1 ? q.bcon[1] : q.bcon[2];
+    const double m = pr[RHO] * ud, eu = eta * ud, m0 = pr[RHO] * q.ucon[0], eu0 = eta * q.ucon[0];
+    x.F[RHO] = m * sg;
+    x.U[RHO] = m0 * sg;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      double t = eu * q.ucov[j];
+      if (j == 1 && d1) t = t + ptot;
+      if (j == 2 && !d1) t = t + ptot;
+      t = t - bd * q.bcov[j];
+      if (!FFDE && j == 0) t = t + m;
+      x.F[UU + j] = t * sg;
+      t = eu0 * q.ucov[j];
+      if (j == 0) t = t + ptot;
+      t = t - q.bcon[0] * q.bcov[j];
+      if (!FFDE && j == 0) t = t + m0;
+      x.U[UU + j] = t * sg;
+    }
+    const double Bd = d1 ? pr[B1] : pr[B2], Bo = d1 ? pr[B2] : pr[B1], uo = d1 ? q.ucon[2] : q.ucon[1];
+    x.F[XB] = ex.div(Bo * ud - Bd * uo, q.ut) * sg;
+    x.F[XB3] = ex.div(pr[B3] * ud - Bd * q.ucon[3], q.ut) * sg;
+    x.U[XB] = Bo * sg;
+    x.U[XB3] = pr[B3] * sg;
+  }
+  // vchar and simplefast
+  const double WW0 = pr[RHO] + gam * pr[UU];
+  const bool wpos = WW0 > 0.;
+  const double WW = wpos ? WW0 : 0.;
+  const double cs2q = Exact::quot(gam * (gam - 1.) * pr[UU], ex.rcp(wpos ? WW0 : 1.));
+  const double cs2 = wpos ? cs2q : 0.;
+  const double EF = q.bsq + WW;
+  const bool epos = EF > 0.;
+  const double va2q = Exact::quot(q.bsq, ex.rcp(epos ? EF : 1.));
+  const double va2 = epos ? va2q : 0.;
+  // numerators unwatched: where the larger of the two squares exceeds 1e-150
+  // its quotient is exact, and one so small that its quotient might not be
+  // leaves cms2 at the other to the last bit (the upper ends are cms2's)
+  ex.need((cs2 > va2 ? cs2 : va2) > 1.e-150);
+  const double cms2 = cs2 + va2 - cs2 * va2;
+  ex.need(cms2 >= 0. && cms2 <= 1.);
+  const double Au = d1 ? q.ucon[1] : q.ucon[2], Bu = q.ucon[0];
+  const double Au2 = Au * Au, Bu2 = Bu * Bu, AuBu = Au * Bu;
+  const double A = Bu2 - (gtt + Bu2) * cms2;
+  const double B = 2. * (AuBu - (gd + AuBu) * cms2);
+  const double C = Au2 - (gdd + Au2) * cms2;
+  const double s = ex.sqrt_of(B * B - 4. * A * C);
+  const Recip A2 = ex.rcp(2. * A);
+  // s >= 2^-100, so neither sum is tiny unless it is zero
+  const double vm = Exact::quot(B - s, A2), vp = Exact::quot(B + s, A2);
+  x.vmax = (vp < vm) ? vm : vp;
+  x.vmin = (vp < vm) ? vp : vm;
+}
+
+// face_flux without branches: left and right point at the two interface
+// states (planes ks doubles apart), dir 1 or 2, base at the metric of the
+// face's location.  F and dtij are valid where ex.ok().
+template <bool FFDE, typename EX>
+__device__ __forceinline__ void face_flux_x(EX& ex, const StepArgs& a, const double* base, int dir, const double* left,
+                                            const double* right, int ks, double* F, double& dtij, int rf)
+{
+  const long long pl = a.gr.plane;
+  double c[10], gcon[4];
+#pragma unroll
+  for (int k = 0; k < 10; k++) c[k] = __ldg(base + k * pl);
+#pragma unroll
+  for (int k = 0; k < 4; k++) gcon[k] = __ldg(base + (10 + k) * pl);
+  const double gdd = __ldg(base + (dir == 1 ? 14 : 17) * pl), sg = __ldg(base + 20 * pl);
+  const double gd = (dir == 1) ? gcon[1] : gcon[2];
+  const double gam = a.pp.gam, limit = (a.pp.gammamax <= 1.) ? 1.e300 : a.pp.gammamax;
+  const int bd = (B1 - 1 + dir) * ks;
+  const double Bd = 0.5 * (left[bd] + right[bd]);
+  const LapseX l = lapse_x(ex, gcon);
+  SideX sl, sr;
+#pragma unroll
+  for (int s = 0; s < 2; s++) {
+    const double* src = s ? right : left;
+    double p[NPR];
+#pragma unroll
+    for (int k = 0; k < NPR; k++) p[k] = src[k * ks];
+    if (dir == 1) p[B1] = Bd;
+    else p[B2] = Bd;
+    StateX q;
+    state_x(ex, p, c, l, limit, q);
+    sl = sr;
+    side_x<FFDE>(ex, p, q, dir, sg, gcon[0], gd, gdd, gam, sr);
+  }
+  double cmin = rmin(sl.vmin, sr.vmin), cmax = rmax(sl.vmax, sr.vmax);
+  cmin = fabs(rmax(0., -cmin));
+  cmax = fabs(rmax(0., cmax));
+  const double ctop = rmax(cmax, cmin), cc = cmax * cmin;
+  const Recip sum = ex.rcp(cmax + cmin);
+  // an in-range divisor keeps both forms finite, so the form that
+  // choose_flux weighs with 0 adds nothing
+#pragma unroll
+  for (int k = 0; k < NX; k++) {
+    const double dU = sr.U[k] - sl.U[k];
+    if (((k < B1) ? rf : a.pp.fluxmethod) == 1) F[k] = ex.div(cmax * sl.F[k] + cmin * sr.F[k] - cc * dU, sum);
+    else F[k] = 0.5 * (sl.F[k] + sr.F[k] - ctop * dU);
+  }
+  dtij = Exact::quot(a.pp.cour * (dir == 1 ? a.pp.dx1 : a.pp.dx2), ex.rcp(ctop));
+}
+
+// fix_flux's face-local rules (fixup.c:1357-1410) on the flux through the
+// face (i, j): the mass-flux sign clamps at the two x1 ends; only u~2's flux
+// crosses the polar and equatorial x2 faces
+template <typename T>
+__device__ __forceinline__ void fix_face(const StepArgs& a, int i, int j, int dir, T* Fo)
+{
+  const int n1 = a.gr.n1, n2 = a.gr.n2;
+  if (dir == 1) {
+    if (i == 0 && a.pp.bc == 0 && j >= -1 && j < n2 && Fo[RHO] > 0) Fo[RHO] = 0;
+    if (i == n1 && j >= -1 && j < n2 && Fo[RHO] < 0) Fo[RHO] = 0;
+  } else {
+    const bool polar = (j == 0 || j == n2) && (i < n1);
+    const bool equator = (j == (n2 - 1) / 2) && (i >= 0) && (i < n1);
+    if (polar || equator) {
+#pragma unroll
+      for (int k = 0; k < NPR; k++)
+        if (k != U2) Fo[k] = T(0.);
+    }
+  }
+}
+
+__device__ __forceinline__ void store_face_x(const StepArgs& a, int i, int j, int dir, long long z, const double* Fx)
+{
+  double Fo[NPR];
+#pragma unroll
+  for (int k = 0; k <= U3; k++) Fo[k] = Fx[k];
+  Fo[B1] = (dir == 1) ? 0. : Fx[XB];
+  Fo[B2] = (dir == 1) ? Fx[XB] : 0.;
+  Fo[B3] = Fx[XB3];
+  fix_face(a, i, j, dir, Fo);
+  double* F = ((dir == 1) ? a.F1 : a.F2) + z;
+#pragma unroll
+  for (int k = 0; k < NPR; k++) F[k * a.gr.plane] = Fo[k];
+}
+
+// The face (i, j) in direction dir that face_flux_x could not take (left: its
+// left state, the right one NPR planes on).  Stores the flux and returns the
+// face's Courant limit.
+template <bool FFDE>
+__device__ __noinline__ double face_general(const StepArgs& a, const double* left, int ks, int i, int j, int dir, int rf)
+{
+  const long long z = a.gr.at(i, j);
+  double pl[NPR], pr[NPR], Fo[NPR], dtij;
+#pragma unroll
+  for (int k = 0; k < NPR; k++) {
+    pl[k] = left[k * ks];
+    pr[k] = left[(NPR + k) * ks];
+  }
+  face_flux<double, FFDE>(a, i, j, dir, pl, pr, Fo, dtij, rf);
+  fix_face(a, i, j, dir, Fo);
+  double* F = ((dir == 1) ? a.F1 : a.F2) + z;
+#pragma unroll
+  for (int k = 0; k < NPR; k++) F[k * a.gr.plane] = Fo[k];
+  return dtij;
+}
+
 __device__ __forceinline__ double block_min(double v, double* sh)
 {
   // exact minimum (no rounding), NaN-ignoring like `if (x < m) m = x`
@@ -133,17 +415,94 @@ __device__ __forceinline__ double block_min(double v, double* sh)
 // two-zone stencil halo on every side and one more row below, for the x2
 // neighbour of its first row -- arrives in shared memory by one TMA copy
 // (flux_tile_*, below); every zone reconstructs its own interface states
-// once from the tile: the x1 neighbour's right state arrives by warp
-// shuffle and the x2 neighbour's through shared memory (the first row
-// recomputes it).  Lane 0's zone is also the previous block's lane 31
-// (blocks step by FLUX_BX = 31 along x1): lane 0 only lends its right state,
-// and its faces are the previous block's (block 0's lane 0 is zone -1,
-// which has no x1 face but an x2 face).
-// BY = 4 or 8 rows per block (flux_rows).  At most 128 registers a thread
-// for the FP64 faces (512 threads per SM), 96 for the FP32 ones (five 4-row
-// blocks per SM).
+// once from the tile (the first row also those of the zones below it).
+// Lane 0's zone is also the previous block's lane 31 (blocks step by FLUX_BX
+// = 31 along x1): lane 0 only lends its right state, and its faces are the
+// previous block's (block 0's lane 0 is zone -1, which has no x1 face but an
+// x2 face).  BY = 4 or 8 rows per block (flux_rows).
+
+// the block's tile: issues its TMA copy (one thread); the zone's value of
+// plane 0 is at the returned pointer
+template <int BY>
+__device__ __forceinline__ const double* flux_tile_load(double* tile, const CUtensorMap* map, uint64_t* bar)
+{
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int cx = (int)(blockIdx.x * FLUX_BX) & ~1;  // the tile's first column (even)
+  if (tx == 0 && ty == 0) {
+    mbar_init(bar, 1);
+    mbar_expect_tx(bar, (uint32_t)flux_tile_bytes(BY));
+    tma_load_3d(tile, map, cx, (int)(blockIdx.y * BY) - 1, 0, bar);
+  }
+  // row ty + 3, column tx + 2 + (the block's first column - cx)
+  return tile + (ty + 3) * FLUX_TILE_W + tx + 2 + ((int)(blockIdx.x * FLUX_BX) - cx);
+}
+
+// the block's Courant minima
+__device__ __forceinline__ void flux_block_dt(const StepArgs& a, double dt1, double dt2, double (*sh)[32])
+{
+  dt1 = block_min(dt1, sh[0]);
+  dt2 = block_min(dt2, sh[1]);
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
+    const int b = blockIdx.y * gridDim.x + blockIdx.x;
+    a.blockmin[b] = dt1;
+    a.blockmin[a.nblocks_flux + b] = dt2;
+  }
+}
+
+// The b^2 flags and the flux choice of the zone at tz, formed in the first
+// substep of a step with the per-zone switch (from the step's p, which is
+// that substep's tile; get_bsqflags, fixup.c:1197-1295, with the b^2 flags
+// the repairs read later): (flags) | (choice) << 8
+__device__ __forceinline__ int flux_flags(const StepArgs& a, const double* tz, int ps, long long z)
+{
+  double pr[NPR];
+#pragma unroll
+  for (int k = 0; k < NPR; k++) pr[k] = tz[k * ps];
+  Geo<double> gz;
+  load_geo(a, CENT, z, gz);
+  unsigned char b = 0;
+  if (!a.pp.eom) {
+    State<double> q;
+    state_of(pr, gz, q);
+    b = bsq_flag(a, pr, q);
+  }
+  const double gamma = gamma_of(pr, gz);
+  const int f1 = (gamma > 2.0 * a.pp.gammadamp) ? 2 : ((gamma > a.pp.gammadamp) ? 1 : 0);
+  const int rf = ((b & 3) == 2 || f1 == 2 || (b >> 2) == 2) ? a.pp.fluxmethod - 1 : a.pp.fluxmethod;
+  return b | ((rf < 0) ? 0 : rf) << 8;
+}
+
+// flux_flags for the FP64 faces: without branches, or flux_flags itself
+static __device__ __noinline__ int flux_flags_x(const StepArgs& a, const double* tz, int ps, long long z)
+{
+  const double* base = a.geo + (long long)CENT * GEO_PER_LOC * a.gr.plane + z;
+  double pr[NPR], c[10], gcon[4];
+#pragma unroll
+  for (int k = 0; k < NPR; k++) pr[k] = tz[k * ps];
+#pragma unroll
+  for (int k = 0; k < 10; k++) c[k] = __ldg(base + k * a.gr.plane);
+#pragma unroll
+  for (int k = 0; k < 4; k++) gcon[k] = __ldg(base + (10 + k) * a.gr.plane);
+  Exact ex;
+  StateX q;
+  state_x(ex, pr, c, lapse_x(ex, gcon), 1.e300, q);
+  const double rl = a.pp.bsqorholimit, ul = a.pp.bsqoulimit;
+  // a tiny b^2's quotients only have to come out below the limits
+  ex.numerator((fabs(q.bsq) < 1.e-200 && rl > 1.e-150 && ul > 1.e-150) ? 0. : q.bsq);
+  const double br = Exact::quot(q.bsq, ex.rcp(pr[RHO])), bu = Exact::quot(q.bsq, ex.rcp(pr[UU]));
+  if (a.pp.eom || !ex.ok()) return flux_flags(a, tz, ps, z);
+  const int f0 = (br > rl) ? 2 : ((br > 0.9 * rl) ? 1 : 0), f3 = (bu > ul) ? 2 : ((bu > 0.9 * ul) ? 1 : 0);
+  const int f1 = (q.gamma > 2.0 * a.pp.gammadamp) ? 2 : ((q.gamma > a.pp.gammadamp) ? 1 : 0);
+  const int rf = (f0 == 2 || f1 == 2 || f3 == 2) ? a.pp.fluxmethod - 1 : a.pp.fluxmethod;
+  return (f0 | (f3 << 2)) | ((rf < 0) ? 0 : rf) << 8;
+}
+
+// FP32 faces (mixed form): both directions through one copy of the face
+// code, dir a run-time value (the direction-dependent reads are selects),
+// which halves the kernel's instruction footprint.  96 registers a thread:
+// five 4-row blocks per SM.
 template <typename T, bool PARA, bool FFDE, int BY>
-__global__ void __launch_bounds__(32 * BY, (sizeof(T) == 8) ? 512 / (32 * BY) : ((BY == FLUX_BY_SMALL) ? 5 : 1))
+__global__ void __launch_bounds__(32 * BY, (BY == FLUX_BY_SMALL) ? 5 : 1)
     k_flux(StepArgs a, const __grid_constant__ CUtensorMap prim_map)
 {
   extern __shared__ __align__(128) double tile[];
@@ -151,13 +510,8 @@ __global__ void __launch_bounds__(32 * BY, (sizeof(T) == 8) ? 512 / (32 * BY) : 
   __shared__ T shr[NPR][BY][32];
   __shared__ uint64_t bar;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  constexpr int ROWS = flux_tile_rows(BY), PS = ROWS * FLUX_TILE_W;
-  const int cx = (int)(blockIdx.x * FLUX_BX) & ~1;  // the tile's first column (even)
-  if (tx == 0 && ty == 0) {
-    mbar_init(&bar, 1);
-    mbar_expect_tx(&bar, (uint32_t)flux_tile_bytes(BY));
-    tma_load_3d(tile, &prim_map, cx, (int)(blockIdx.y * BY) - 1, 0, &bar);
-  }
+  constexpr int PS = flux_tile_rows(BY) * FLUX_TILE_W;
+  const double* tz = flux_tile_load<BY>(tile, &prim_map, &bar);
   const int i = blockIdx.x * FLUX_BX + tx - 1;
   const int j = blockIdx.y * BY + ty - 1;
   const int n1 = a.gr.n1, n2 = a.gr.n2;
@@ -175,153 +529,203 @@ __global__ void __launch_bounds__(32 * BY, (sizeof(T) == 8) ? 512 / (32 * BY) : 
     if (tx == 0 && ty == 0) report_fail(a.sc, a.phase0 + PH_FACE1, FAIL_TMA_TIMEOUT, zone_order(i, j));
     return;
   }
-  // the zone's value of plane 0 in the tile: row ty + 3, column tx + 2 + (the
-  // block's first column - cx)
-  const double* tz = tile + (ty + 3) * FLUX_TILE_W + tx + 2 + ((int)(blockIdx.x * FLUX_BX) - cx);
   // the flux choice of this zone, which both of its faces use: fluxmethod,
-  // or with the per-zone switch FLAGREALFLUX, formed here in the first
-  // substep of the FP64 step (from the step's p, which is this substep's
-  // tile; get_bsqflags, fixup.c:1197-1295, with the b^2 flags the repairs
-  // read later) and read back in the second
+  // or with the per-zone switch FLAGREALFLUX, formed in the first substep
+  // and read back in the second
   int rf = a.pp.fluxmethod;
   if (a.pp.fluxadjust && in) {
     if (a.flags_here) {
-      double pr[NPR];
-#pragma unroll
-      for (int k = 0; k < NPR; k++) pr[k] = tz[k * PS];
-      Geo<double> gz;
-      load_geo(a, CENT, z, gz);
-      unsigned char b = 0;
-      if (!a.pp.eom) {
-        State<double> q;
-        state_of(pr, gz, q);
-        b = bsq_flag(a, pr, q);
-      }
-      const double gamma = gamma_of(pr, gz);
-      const int f1 = (gamma > 2.0 * a.pp.gammadamp) ? 2 : ((gamma > a.pp.gammadamp) ? 1 : 0);
-      rf = ((b & 3) == 2 || f1 == 2 || (b >> 2) == 2) ? a.pp.fluxmethod - 1 : a.pp.fluxmethod;
-      rf = (rf < 0) ? 0 : rf;
+      const int f = flux_flags(a, tz, PS, z);
+      rf = f >> 8;
       if (own) {
-        a.bsqf[z] = b;
+        a.bsqf[z] = (unsigned char)(f & 255);
         a.fluxf[z] = (unsigned char)rf;
       }
     } else {
       rf = (int)a.fluxf[z];
     }
   }
-  if constexpr (sizeof(T) == 4) {
-    // FP32 faces (mixed form): both directions through one copy of the face
-    // code, dir a run-time value (the direction-dependent reads are
-    // selects), which halves the kernel's instruction footprint (the FP32
-    // kernel stalls on instruction fetch: 1% on the mixed step).  The FP64
-    // faces keep one copy per direction (below): the shared copy's register
-    // allocation cost them 0.3%.
 #pragma unroll 1
-    for (int dir = 1; dir <= 2; dir++) {
-      zone_states<T, PARA>(tz, PS, (dir == 1) ? 1 : FLUX_TILE_W, L, R);
-      bool act;
-      if (dir == 1) {
+  for (int dir = 1; dir <= 2; dir++) {
+    zone_states<T, PARA>(tz, PS, (dir == 1) ? 1 : FLUX_TILE_W, L, R);
+    bool act;
+    if (dir == 1) {
 #pragma unroll
-        for (int k = 0; k < NPR; k++) pl[k] = __shfl_up_sync(0xffffffffu, R[k], 1);
-        act = in && i >= 0 && tx > 0;
-      } else {
-#pragma unroll
-        for (int k = 0; k < NPR; k++) shr[k][ty][tx] = R[k];
-        __syncthreads();
-        if (ty > 0) {
-#pragma unroll
-          for (int k = 0; k < NPR; k++) pl[k] = shr[k][ty - 1][tx];
-        } else {
-          T Lm[NPR];
-          zone_states<T, PARA>(tz - FLUX_TILE_W, PS, FLUX_TILE_W, Lm, pl);
-        }
-        act = in && j >= 0 && own;
-      }
-      if (act) {
-        face_flux<T, FFDE>(a, i, j, dir, pl, L, Fo, dtij, rf);
-        T* F;
-        if (dir == 1) {
-          // x1: fix_flux's mass-flux sign clamps at the two ends
-          dt1 = (dtij < dt1) ? dtij : dt1;
-          if (i == 0 && a.pp.bc == 0 && j >= -1 && j < n2 && Fo[RHO] > 0) Fo[RHO] = 0;
-          if (i == n1 && j >= -1 && j < n2 && Fo[RHO] < 0) Fo[RHO] = 0;
-          F = F1;
-        } else {
-          // x2: only u~2's flux crosses the polar and equatorial faces
-          dt2 = (dtij < dt2) ? dtij : dt2;
-          const bool polar = (j == 0 || j == n2) && (i < n1);
-          const bool equator = (j == (n2 - 1) / 2) && (i >= 0) && (i < n1);
-          if (polar || equator) {
-#pragma unroll
-            for (int k = 0; k < NPR; k++)
-              if (k != U2) Fo[k] = T(0.);
-          }
-          F = F2;
-        }
-#pragma unroll
-        for (int k = 0; k < NPR; k++) F[k * a.gr.plane + z] = Fo[k];
-      }
-    }
-  } else {
-    // ---- x1 faces
-    zone_states<T, PARA>(tz, PS, 1, L, R);
-#pragma unroll
-    for (int k = 0; k < NPR; k++) pl[k] = __shfl_up_sync(0xffffffffu, R[k], 1);
-    if (in && i >= 0 && tx > 0) {
-      face_flux<T, FFDE>(a, i, j, 1, pl, L, Fo, dtij, rf);
-      dt1 = (dtij < dt1) ? dtij : dt1;
-      if (i == 0 && a.pp.bc == 0 && j >= -1 && j < n2 && Fo[RHO] > 0) Fo[RHO] = 0;
-      if (i == n1 && j >= -1 && j < n2 && Fo[RHO] < 0) Fo[RHO] = 0;
-#pragma unroll
-      for (int k = 0; k < NPR; k++) F1[k * a.gr.plane + z] = Fo[k];
-    }
-    // ---- x2 faces
-    zone_states<T, PARA>(tz, PS, FLUX_TILE_W, L, R);
-#pragma unroll
-    for (int k = 0; k < NPR; k++) shr[k][ty][tx] = R[k];
-    __syncthreads();
-    if (ty > 0) {
-#pragma unroll
-      for (int k = 0; k < NPR; k++) pl[k] = shr[k][ty - 1][tx];
+      for (int k = 0; k < NPR; k++) pl[k] = __shfl_up_sync(0xffffffffu, R[k], 1);
+      act = in && i >= 0 && tx > 0;
     } else {
-      T Lm[NPR];
-      zone_states<T, PARA>(tz - FLUX_TILE_W, PS, FLUX_TILE_W, Lm, pl);
-    }
-    if (in && j >= 0 && own) {
-      face_flux<T, FFDE>(a, i, j, 2, pl, L, Fo, dtij, rf);
-      dt2 = (dtij < dt2) ? dtij : dt2;
-      const bool polar = (j == 0 || j == n2) && (i < n1);
-      const bool equator = (j == (n2 - 1) / 2) && (i >= 0) && (i < n1);
-      if (polar || equator) {
 #pragma unroll
-        for (int k = 0; k < NPR; k++)
-          if (k != U2) Fo[k] = T(0.);
+      for (int k = 0; k < NPR; k++) shr[k][ty][tx] = R[k];
+      __syncthreads();
+      if (ty > 0) {
+#pragma unroll
+        for (int k = 0; k < NPR; k++) pl[k] = shr[k][ty - 1][tx];
+      } else {
+        T Lm[NPR];
+        zone_states<T, PARA>(tz - FLUX_TILE_W, PS, FLUX_TILE_W, Lm, pl);
       }
+      act = in && j >= 0 && own;
+    }
+    if (act) {
+      face_flux<T, FFDE>(a, i, j, dir, pl, L, Fo, dtij, rf);
+      T* F;
+      if (dir == 1) {
+        dt1 = (dtij < dt1) ? dtij : dt1;
+        F = F1;
+      } else {
+        dt2 = (dtij < dt2) ? dtij : dt2;
+        F = F2;
+      }
+      fix_face(a, i, j, dir, Fo);
 #pragma unroll
-      for (int k = 0; k < NPR; k++) F2[k * a.gr.plane + z] = Fo[k];
+      for (int k = 0; k < NPR; k++) F[k * a.gr.plane + z] = Fo[k];
     }
   }
-  dt1 = block_min(dt1, sh[0]);
-  dt2 = block_min(dt2, sh[1]);
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    const int b = blockIdx.y * gridDim.x + blockIdx.x;
-    a.blockmin[b] = dt1;
-    a.blockmin[a.nblocks_flux + b] = dt2;
+  flux_block_dt(a, dt1, dt2, sh);
+}
+
+// FP64 faces.  FP64 issue and latency bound: 2080 FP64-pipe instructions a
+// zone at 128 registers (16 warps per SM).  What the layout is for:
+//  * all interface states are formed first, into shared memory (four slots a
+//    zone: the left and right state of its x1 and x2 face).  A warp takes one
+//    variable of the whole block and walks along the zones, so each slope and
+//    raw interface value is formed once (93 instead of 172 FP64 instructions
+//    a variable and zone), and the block meets at one barrier while its warps
+//    are still together;
+//  * then each thread takes its two faces in one stretch of code without a
+//    branch (harm_exact.cuh).  Warps with states so small that quotients
+//    leave Exact's range (the field ahead of its front: 5% of the warps of
+//    the 512^2 torus at t = 3, 13% of the 1024^2 one at t = 0.8) take the
+//    ExactTiny form, and what neither can take goes to face_general, whose
+//    code is cold: 0.2% of the warps there cost 20% of the kernel.
+// Time per launch, developed flow, mean of both substeps (one face at a time,
+// each quotient and root with its own branches -> this form): 512^2 PARA
+// with the switch 152 -> 88 us, 1024^2 626 -> 299 us, 128^2 MC 26 -> 16 us,
+// the force-free 512 x 256 dipole 63.5 -> 38 us.
+// a row of a slot plane: 33 doubles, so that lanes in successive rows hit
+// successive banks
+constexpr int FLUX_SLOT_W = 33;
+template <bool PARA, bool FFDE, int BY>
+__global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
+    k_flux_fp64(const __grid_constant__ StepArgs a, const __grid_constant__ CUtensorMap prim_map)
+{
+  extern __shared__ __align__(128) double tile[];
+  __shared__ double sh[2][32];
+  __shared__ uint64_t bar;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  constexpr int PS = flux_tile_rows(BY) * FLUX_TILE_W, SW = FLUX_SLOT_W, KS = BY * SW;
+  const double* tz = flux_tile_load<BY>(tile, &prim_map, &bar);
+  double* slot = tile + NPR * PS + ty * SW + tx;  // state s of direction dir: slot[(2 * dir - 2 + s) * NPR * KS + k * KS]
+  const int i = blockIdx.x * FLUX_BX + tx - 1;
+  const int j = blockIdx.y * BY + ty - 1;
+  const int n1 = a.gr.n1, n2 = a.gr.n2;
+  const bool in = (i <= n1) && (j <= n2);
+  const bool own = (tx > 0) || (blockIdx.x == 0);  // lane 0 of a later block repeats a zone
+  const long long z = a.gr.at(in ? i : -1, in ? j : -1);
+  double dt1 = 1.e9, dt2 = 1.e9;
+  __syncthreads();  // the barrier is initialised before anyone polls it
+  if (!mbar_wait(&bar, 0)) {
+    if (tx == 0 && ty == 0) report_fail(a.sc, a.phase0 + PH_FACE1, FAIL_TMA_TIMEOUT, zone_order(i, j));
+    return;
   }
+  // a warp forms the states of one variable (BY = 8) or two at all of the
+  // block's zones: along x2 a lane per column (and the zones below the first
+  // row, for their right states), along x1 a lane per BY zones of a row.  A
+  // zone's right state is the left state of the next zone's face.
+#pragma unroll 1
+  for (int k = ty; k < NPR; k += BY) {
+    const double* t = tz + (k * PS - ty * FLUX_TILE_W - tx);  // the block's first zone
+    double* d = slot + (k * KS - ty * SW - tx);
+    {
+      double* d2 = d + 2 * NPR * KS + tx;
+      row_states<PARA, BY + 1>(t + tx - FLUX_TILE_W, FLUX_TILE_W, [&](int c, double l, double r) {
+        if (c > 0) d2[NPR * KS + (c - 1) * SW] = l;
+        if (c < BY) d2[c * SW] = r;
+      });
+    }
+    const int row = tx % BY, c0 = (tx / BY) * BY;
+    d += row * SW + c0;
+    row_states<PARA, BY>(t + row * FLUX_TILE_W + c0, 1, [&](int c, double l, double r) {
+      d[NPR * KS + c] = l;
+      d[c + 1] = r;  // (the last zone's goes to the row's padding)
+    });
+  }
+  // the flux choice of this zone (as in k_flux)
+  int rf = a.pp.fluxmethod;
+  if (a.pp.fluxadjust && in) {
+    if (a.flags_here) {
+      const int f = flux_flags_x(a, tz, PS, z);
+      rf = f >> 8;
+      if (own) {
+        a.bsqf[z] = (unsigned char)(f & 255);
+        a.fluxf[z] = (unsigned char)rf;
+      }
+    } else {
+      rf = (int)a.fluxf[z];
+    }
+  }
+  __syncthreads();
+  // whether one of the states of the warp's faces holds a velocity or field
+  // so small that quotients may leave Exact's range
+  bool small = false;
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int k = U1; k <= B3; k++) {
+      // (volatile: these values are read again where they are used)
+      const double v = *const_cast<const volatile double*>(slot + (q * NPR + k) * KS);
+      const uint32_t t = hi_word(v) & 0x7fffffffu;
+      small |= (t < Exact::word(-850)) && ((t | lo_word(v)) != 0);
+    }
+  const bool tiny = __any_sync(0xffffffffu, small);
+  // both faces in one stretch of code; what it could not take comes after it
+  bool todo1 = in && i >= 0 && tx > 0, todo2 = in && j >= 0 && own;
+  auto faces = [&](auto ex0) {
+#pragma unroll
+    for (int dir = 1; dir <= 2; dir++) {
+      bool& todo = (dir == 1) ? todo1 : todo2;
+      if (!todo) continue;
+      const double* left = slot + (2 * dir - 2) * NPR * KS;
+      const double* base = a.geo + (long long)(dir == 1 ? FACE1 : FACE2) * GEO_PER_LOC * a.gr.plane + z;
+      double Fx[NX], dtij;
+      auto ex = ex0;
+      face_flux_x<FFDE>(ex, a, base, dir, left, left + NPR * KS, KS, Fx, dtij, rf);
+      if (ex.ok()) {
+        store_face_x(a, i, j, dir, z, Fx);
+        if (dir == 1) dt1 = (dtij < dt1) ? dtij : dt1;
+        else dt2 = (dtij < dt2) ? dtij : dt2;
+        todo = false;
+      }
+    }
+  };
+  if (!tiny) faces(Exact());
+  else faces(ExactTiny());
+#pragma unroll 1
+  for (int dir = 1; dir <= 2; dir++) {
+    if (!((dir == 1) ? todo1 : todo2)) continue;
+    const double dtij = face_general<FFDE>(a, slot + (2 * dir - 2) * NPR * KS, KS, i, j, dir, rf);
+    if (dir == 1) dt1 = (dtij < dt1) ? dtij : dt1;
+    else dt2 = (dtij < dt2) ? dtij : dt2;
+  }
+  flux_block_dt(a, dt1, dt2, sh);
 }
 
 // the k_flux instance of the block's row count (b.y); its dynamic shared
-// memory limit raised once to the tile's size
+// memory limit raised once to its size
 template <typename T, bool PARA, bool FFDE, int BY>
 inline void flux_launch_by(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map)
 {
-  constexpr size_t sm = flux_tile_bytes(BY);
+  constexpr bool fp64 = sizeof(T) == 8;
+  constexpr size_t sm = flux_tile_bytes(BY) + (fp64 ? 4 * NPR * BY * FLUX_SLOT_W * sizeof(double) : 0);
+  void (*kern)(StepArgs, CUtensorMap);
+  if constexpr (fp64) kern = k_flux_fp64<PARA, FFDE, BY>;
+  else kern = k_flux<T, PARA, FFDE, BY>;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_flux<T, PARA, FFDE, BY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     attr = true;
   }
-  k_flux<T, PARA, FFDE, BY><<<g, b, sm, s>>>(a, map);
+  kern<<<g, b, sm, s>>>(a, map);
 }
 template <typename T, bool PARA, bool FFDE>
 inline void flux_rows_launch(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map)

@@ -1,0 +1,62 @@
+"""The branch-free quotients and roots of the FP64 kernels (harm_exact.cuh)
+round as IEEE division and square root do: equal to the operators for every
+operand reported in range, on the host with seeds a few units off and on the
+device with its own approximations; operands out of range are reported."""
+import shutil
+
+import numpy as np
+import pytest
+
+import exact_cases as ec
+
+needs_nvcc = pytest.mark.skipif(shutil.which("/usr/local/cuda/bin/nvcc") is None, reason="needs nvcc")
+PLACES = [pytest.param("host", n, marks=needs_nvcc) for n in (1, 2, 3)] + [
+    pytest.param("device", 0, marks=pytest.mark.gpu)]
+
+
+@pytest.mark.parametrize("where,nudge", PLACES)
+def test_quotients(where, nudge):
+    for name, a, b in ec.operand_sets():
+        q, ok = ec.evaluate(where, False, a, b, nudge)
+        assert ok.all(), name
+        assert np.array_equal(q, a / b), name
+
+
+@pytest.mark.parametrize("where,nudge", PLACES)
+def test_quotients_of_tiny_numbers(where, nudge):
+    r = np.random.default_rng(9)
+    n = 1 << 20
+    a, b = ec.hard_quotients(500)
+    sets = [(a * 2.0 ** -60, b)]
+    # numerators and quotients across the subnormal range, and exact ties of it
+    sets += [(a * 2.0 ** -k, b * 2.0 ** s) for k in range(1075, 1130, 3) for s in (-1, 0, 1, 5)]
+    sets += [(r.uniform(1, 2, n) * 2.0 ** r.integers(-1074, -960, n), r.uniform(1, 2, n) * 2.0 ** r.integers(-40, 40, n))]
+    sets += [(r.integers(-4000, 4000, n) * 5e-324, r.integers(1, 64, n).astype(float))]
+    sets += [(r.uniform(1, 2, n) * 2.0 ** r.integers(-960, 190, n), r.uniform(1, 2, n) * 2.0 ** r.integers(-200, 60, n))]
+    for a, b in sets:
+        q, ok = ec.evaluate(where, 2, a, b, nudge)
+        assert ok.all()
+        assert np.array_equal(q, a / b)
+
+
+@pytest.mark.parametrize("where,nudge", PLACES)
+def test_roots(where, nudge):
+    hard = ec.hard_roots()
+    assert len(hard) > 80
+    r = np.random.default_rng(8)
+    n = 1 << 20
+    for x in (hard, hard * 4.0 ** -33, hard * 4.0 ** 28, r.uniform(1, 4, n), r.uniform(1, 2, n) * 2.0 ** r.integers(-200, 60, n),
+              1.0 + 2.0 ** -52 * np.arange(1000)):
+        q, ok = ec.evaluate(where, True, x, x, nudge)
+        assert ok.all()
+        assert np.array_equal(q, np.sqrt(x))
+
+
+@pytest.mark.parametrize("where,nudge", PLACES[-2:])
+def test_out_of_range_is_reported(where, nudge):
+    tiny = np.array([5e-324, 2.0 ** -1022, 2.0 ** -951, np.inf, -np.inf, np.nan, 2.0 ** 601])
+    assert not ec.evaluate(where, False, tiny, np.ones(len(tiny)), nudge)[1].any()
+    wild = np.array([0.0, -0.0, -1.0, 5e-324, 2.0 ** -201, 2.0 ** 61, np.inf, np.nan, -np.inf])
+    assert not ec.evaluate(where, False, np.ones(len(wild)), wild, nudge)[1].any()
+    wild = np.array([0.0, -0.0, -1.0, 5e-324, 2.0 ** -201, 2.0 ** 61, np.inf, np.nan])
+    assert not ec.evaluate(where, True, wild, wild, nudge)[1].any()
