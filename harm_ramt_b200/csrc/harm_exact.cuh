@@ -132,6 +132,12 @@ struct Exact {
     const double e1 = fma(-b, y1, 1.0);
     return Recip{b, fma(y1, e1 + 0x1p-95, y1)};
   }
+  // the reciprocal of b from a value y1 within 2^-51 of it
+  HD_INLINE Recip rcp_from(double b, double y1)
+  {
+    pos = above(pos, hi_word(b), word(POS_LO));
+    return Recip{b, fma(y1, fma(-b, y1, 1.0) + 0x1p-95, y1)};
+  }
   // a / d.b for a numerator known to be in range (or zero)
   static HD_INLINE double quot(double a, const Recip& d)
   {

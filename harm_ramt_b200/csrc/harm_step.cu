@@ -61,6 +61,21 @@ __global__ void k_bsqflags(StepArgs a, const double* __restrict__ pv)
   }
 }
 
+// utoprim_2d to its full iteration limit: without branches, or itself
+__device__ __forceinline__ int utoprim_2d_full(const double* U, const Geo<double>& g, double* pr, double gam,
+                                               double gammafail, int* niter, double* nst, long long nss, bool resume)
+{
+  double p[NPR];
+#pragma unroll
+  for (int k = 0; k < NPR; k++) p[k] = pr[k];
+  ExactTiny ex;
+  const int pfl = utoprim_2d_x(ex, U, g.gcov, g.gcon, g.g, p, gam, gammafail, niter, 200, nst, nss, resume);
+  if (!ex.ok()) return utoprim_2d(U, g, pr, gam, gammafail, niter, 200, nst, nss, resume);
+#pragma unroll
+  for (int k = 0; k < NPR; k++) pr[k] = p[k];
+  return pfl;
+}
+
 // The deferred inversions of k_update, continued from the Newton state
 // k_update saved (repair scratch planes 0-4) up to the full iteration limit.
 // A deferred zone's pf slot was not written, so pi still holds its guess.
@@ -85,7 +100,7 @@ __global__ void __launch_bounds__(64) k_update_tail(StepArgs a, const double* __
     int niter;
     double* nst = a.fixbuf + z;
     const bool resume = nst[(NEWTON_STATE - 1) * pl] >= 0.0;
-    int pfl = utoprim_2d(U, g, pfz, a.pp.gam, a.pp.gammafail, &niter, 200, nst, pl, resume);
+    int pfl = utoprim_2d_full(U, g, pfz, a.pp.gam, a.pp.gammafail, &niter, nst, pl, resume);
     if (TA && pfl != 0) {
       double pr0[NPR];
 #pragma unroll
@@ -119,7 +134,7 @@ __global__ void k_invert_zones(StepArgs a, int which, int nz, const int* __restr
   int code;
   if (which == ta::M_2D || which < 0) {
     int niter;
-    code = utoprim_2d(u, g, p, a.pp.gam, a.pp.gammafail, &niter);
+    code = utoprim_2d_full(u, g, p, a.pp.gam, a.pp.gammafail, &niter, nullptr, 0, false);
     if (which < 0) code = ta::tryagain_chain(u, g, a.pp.gam, a.pp.gammafail, p0, p, code);
   } else {
     double Ug[NPR];

@@ -209,6 +209,36 @@ __device__ __forceinline__ void state_x(EX& ex, const double* pr, const double* 
   q.bsq = dot4(q.bcon, q.bcov);
 }
 
+// primtoflux in time: the conserved vector
+template <bool FFDE>
+__device__ __forceinline__ void conserved_x(const double* pr, const StateX& q, double sg, double gam, double* U)
+{
+  const double r = FFDE ? 0. : pr[RHO], u = FFDE ? 0. : pr[UU], P = (gam - 1.) * u, w = P + r + u;
+  const double eta = FFDE ? q.bsq : w + q.bsq, ptot = FFDE ? q.bsq * 0.5 : P + q.bsq * 0.5;
+  const double m = pr[RHO] * q.ucon[0], eu = eta * q.ucon[0];
+  U[RHO] = m * sg;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    double t = eu * q.ucov[j];
+    if (j == 0) t = t + ptot;
+    t = t - q.bcon[0] * q.bcov[j];
+    if (!FFDE && j == 0) t = t + m;
+    U[UU + j] = t * sg;
+  }
+#pragma unroll
+  for (int k = B1; k <= B3; k++) U[k] = pr[k] * sg;
+}
+
+// bsq_flag (a tiny b^2's quotients only have to come out below the limits)
+__device__ __forceinline__ unsigned char bsq_flag_x(Exact& ex, const StepArgs& a, const double* pr, double bsq)
+{
+  const double rl = a.pp.bsqorholimit, ul = a.pp.bsqoulimit;
+  ex.numerator((fabs(bsq) < 1.e-200 && rl > 1.e-150 && ul > 1.e-150) ? 0. : bsq);
+  const double br = Exact::quot(bsq, ex.rcp(pr[RHO])), bu = Exact::quot(bsq, ex.rcp(pr[UU]));
+  const int f0 = (br > rl) ? 2 : ((br > 0.9 * rl) ? 1 : 0), f3 = (bu > ul) ? 2 : ((bu > 0.9 * ul) ? 1 : 0);
+  return (unsigned char)(f0 | (f3 << 2));
+}
+
 // What a face takes from one interface state.  The B^dir row of the flux and
 // of the conserved vectors' difference is zero on both sides (B^dir is
 // continuous), so two field components are kept: the other one of the plane
@@ -486,15 +516,11 @@ static __device__ __noinline__ int flux_flags_x(const StepArgs& a, const double*
   Exact ex;
   StateX q;
   state_x(ex, pr, c, lapse_x(ex, gcon), 1.e300, q);
-  const double rl = a.pp.bsqorholimit, ul = a.pp.bsqoulimit;
-  // a tiny b^2's quotients only have to come out below the limits
-  ex.numerator((fabs(q.bsq) < 1.e-200 && rl > 1.e-150 && ul > 1.e-150) ? 0. : q.bsq);
-  const double br = Exact::quot(q.bsq, ex.rcp(pr[RHO])), bu = Exact::quot(q.bsq, ex.rcp(pr[UU]));
+  const unsigned char b = bsq_flag_x(ex, a, pr, q.bsq);
   if (a.pp.eom || !ex.ok()) return flux_flags(a, tz, ps, z);
-  const int f0 = (br > rl) ? 2 : ((br > 0.9 * rl) ? 1 : 0), f3 = (bu > ul) ? 2 : ((bu > 0.9 * ul) ? 1 : 0);
   const int f1 = (q.gamma > 2.0 * a.pp.gammadamp) ? 2 : ((q.gamma > a.pp.gammadamp) ? 1 : 0);
-  const int rf = (f0 == 2 || f1 == 2 || f3 == 2) ? a.pp.fluxmethod - 1 : a.pp.fluxmethod;
-  return (f0 | (f3 << 2)) | ((rf < 0) ? 0 : rf) << 8;
+  const int rf = ((b & 3) == 2 || f1 == 2 || (b >> 2) == 2) ? a.pp.fluxmethod - 1 : a.pp.fluxmethod;
+  return b | ((rf < 0) ? 0 : rf) << 8;
 }
 
 // FP32 faces (mixed form): both directions through one copy of the face
@@ -803,95 +829,307 @@ __device__ __forceinline__ void finish_zone(const StepArgs& a, const Geo<double>
   for (int k = 0; k < NPR; k++) pf[k * pl + z] = pfz[k];
 }
 
-// advance_standard zone loop, advance.c:114-181, for one RK2 substep.
-// CUf = {1, 0, c2}: Uf = Ui + c2*dt*dU; on the last substep unew = Uf.
-// The connection coefficients and floors arrive by TMA (geo_map, a 3D map
-// over the geometry block with the box above) while U(p_i) and the flux
-// divergence are formed from global loads; the block width is even.
-template <typename FT, bool FFDE>
-__global__ void __launch_bounds__(128, 4) k_update(StepArgs a, const __grid_constant__ CUtensorMap geo_map,
-                                                const double* __restrict__ pi, const double* __restrict__ pb,
-                                                double* __restrict__ pf, double c2)
+// ---- the zone update without branches (harm_exact.cuh)
+// utoprim_2d (harm_device.cuh) with the same operands in the same order,
+// every quotient and root through `ex`; its rare exits (a bad guess, an
+// iterate out of bounds) leave ex.ok() false.  The result, pflag and iteration
+// count hold where ex.ok().
+//
+// Numerators of the Newton step are not watched.  Q.B^2 may be arbitrarily
+// small, but a W in range keeps the terms with it below 2^-700 where its
+// quotients are not exact, and there they change nothing to the last bit:
+// they are added to terms of order W or W^2, to a residual that is zero or
+// larger, or to a vsq that is zero (the new vsq is then below the range that
+// its reciprocal is watched for) or at least 2^-200.  A dx whose own quotient
+// is not exact is far below the tolerance either way.
+__device__ __forceinline__ double utsq_calc_x(ExactTiny& ex, const U2PCtx& c, double W)
 {
-  extern __shared__ __align__(128) double sgeo[];
-  __shared__ uint64_t bar;
+  const double Wsq = W * W, W4 = Wsq * Wsq;
+  const double den = W4 + 2. * c.Bsq * Wsq * W + Wsq * (c.Bsq * c.Bsq - c.Qtsq) - c.QdotBsq * (2. * W + c.Bsq);
+  return ex.Exact::div(c.Bsq * c.QdotBsq + W * (2. * c.QdotBsq + c.Qtsq * W), ex.rcp(den));
+}
+
+__device__ __forceinline__ int newton_vsq_x(ExactTiny& ex, const U2PCtx& c, double& x0, double& x1, double gammafail,
+                                            int& niter_out, int maxit, double* st, long long ss, bool resume)
+{
+  constexpr int MAX_NEWT_ITER = 200;
+  constexpr double NEWT_TOL = 1.0e-15, MIN_NEWT_TOL = 1.0e-10, W_TOO_BIG = 1.e9;
+  const double vsq_too_big = (1.0 - 1.0 / (gammafail - 1.0));
+  const double Bsq = c.Bsq, QdotBsq = c.QdotBsq, gam = c.gam;
+  double errx = 1., errx_old = 2., errx_oldest;
+  int n_iter = 0;
+  if (resume) {
+    x0 = st[0];
+    x1 = st[ss];
+    errx = st[2 * ss];
+    errx_old = st[3 * ss];
+    n_iter = (int)st[4 * ss];
+  }
+  const Recip rgam = ex.rcp(gam), rwg = ex.rcp(c.wglobal);
+  Recip rW = ex.rcp(x0);
+#pragma unroll 1
+  while ((errx > NEWT_TOL) && (n_iter < maxit)) {
+    // func_vsq
+    const double W = x0, vsq = x1, Wsq = W * W, W3 = Wsq * W, gtmp = 1. - vsq;
+    const double sq = ex.sqrt_of(gtmp);
+    const Recip r2 = ex.rcp_from(Wsq, rW.y * rW.y), r3 = ex.rcp_from(W3, r2.y * rW.y);
+    const double p_tmp = Exact::quot((gam - 1.) * (W * gtmp - c.D * sq), rgam);
+    const double dPdW = Exact::quot((gam - 1.) * gtmp, rgam);
+    const double dPdvsq = Exact::quot((gam - 1.) * (Exact::quot(0.5 * c.D, ex.rcp(sq)) - W), rgam);
+    const double BW = Bsq + W;
+    const double t2 = c.Qtsq - vsq * (BW * BW) + Exact::quot(QdotBsq * (Bsq + 2 * W), r2);
+    const double t3 = c.Qdotn - (Bsq * (1 + vsq)) / 2. + 0.5 * Exact::quot(QdotBsq, r2) - W + p_tmp;
+    const double QW3 = Exact::quot(QdotBsq, r3), s = -1 + dPdW - QW3;
+    double dx0 = (-Bsq / 2. + dPdvsq) * t2 + (BW * BW) * t3;
+    double dx1 = -(s * t2) - 2 * (vsq + QW3) * BW * t3;
+    const double detJ = BW * (s * BW + Exact::quot((Bsq - 2 * dPdvsq) * (QdotBsq + vsq * W3), r3));
+    const Recip rd = ex.rcp(fabs(detJ));
+    dx0 = Exact::quot((detJ < 0.) ? dx0 : -dx0, rd);
+    dx1 = Exact::quot((detJ < 0.) ? dx1 : -dx1, rd);
+    if (((n_iter + 1) % 10) == 0) {
+      const double r = cycle_break_uniform(x0, x1, n_iter);
+      dx0 *= r;
+      dx1 *= r;
+    }
+    errx_oldest = errx_old;
+    errx_old = errx;
+    x0 = fabs(x0 + dx0);
+    rW = ex.rcp(x0);
+    x1 += dx1;
+    // where x1 is zero the reference takes |dx1| itself
+    errx = (Exact::quot(fabs(dx0), rW) + Exact::quot(fabs(dx1), ex.rcp((x1 == 0.) ? 1. : fabs(x1)))) / 2.;
+    ex.need(!(Exact::quot(x0, rwg) > W_TOO_BIG));
+    x1 = (x1 < 0.) ? 0.0 : x1;
+    x1 = (x1 > 1.) ? vsq_too_big : x1;
+    if (((errx_old == errx) || (errx_oldest == errx)) && (errx < MIN_NEWT_TOL)) errx = -errx;
+    n_iter++;
+  }
+  niter_out = n_iter;
+  if (maxit < MAX_NEWT_ITER && n_iter >= maxit && errx > NEWT_TOL) {
+    if (st && ex.ok()) {
+      st[0] = x0;
+      st[ss] = x1;
+      st[2 * ss] = errx;
+      st[3 * ss] = errx_old;
+      st[4 * ss] = (double)n_iter;
+    }
+    return NEWTON_DEFERRED;
+  }
+  if (n_iter >= MAX_NEWT_ITER) return (errx > MIN_NEWT_TOL) ? 1 : 0;
+  return 0;
+}
+
+// c, gn: the packed g_{mu nu} and g^{mu nu}; sg: sqrt(-g)
+__device__ __forceinline__ int utoprim_2d_x(ExactTiny& ex, const double* U, const double* c, const double* gn, double sg,
+                                            double* pr, double gam, double gammafail, int* niter, int maxit, double* nst,
+                                            long long nss, bool resume)
+{
+  constexpr double W_TOO_BIG = 1.e9, FAIL_VAL = 1.e30;
+  double Ut[NPR];
+  const Recip rs = ex.rcp(sg);
+  const double ngn = -gn[0];
+  const Recip ral = ex.rcp(Exact::quot(1., ex.rcp(ex.sqrt_of(ngn))));  // alpha
+  const double alpha = ral.b;
+  {
+    double Ug[NPR];
+#pragma unroll
+    for (int k = 0; k < B1; k++) Ug[k] = ex.Exact::div(U[k], rs);
+#pragma unroll
+    for (int k = B1; k <= B3; k++) Ug[k] = ex.div(U[k], rs);
+    Ug[UU] += -Ug[RHO];
+    Ut[RHO] = Ug[RHO] * alpha;
+#pragma unroll
+    for (int k = UU; k <= U3; k++) Ut[k] = -alpha * Ug[k];
+#pragma unroll
+    for (int k = B1; k <= B3; k++) Ut[k] = alpha * Ug[k];
+  }
+  const double* B = Ut + B1;
+  const double* Q = Ut + UU;
+  U2PCtx x;
+  x.gam = gam;
+  const double Bv1 = c[4] * B[0] + c[5] * B[1] + c[6] * B[2], Bv2 = c[5] * B[0] + c[7] * B[1] + c[8] * B[2];
+  const double Bv3 = c[6] * B[0] + c[8] * B[1] + c[9] * B[2];
+  x.Bsq = B[0] * Bv1 + B[1] * Bv2 + B[2] * Bv3;
+  double Qcon[4];
+  lower_v(Q, gn, Qcon);
+  const double QdotB = Q[1] * B[0] + Q[2] * B[1] + Q[3] * B[2];
+  x.QdotBsq = QdotB * QdotB;
+  const double nlapse = -ex.sqrt_of(Exact::quot(1., ex.rcp(ngn)));
+  x.Qdotn = Qcon[0] * nlapse;
+  x.Qtsq = Q[0] * Qcon[0] + Q[1] * Qcon[1] + Q[2] * Qcon[2] + Q[3] * Qcon[3] + x.Qdotn * x.Qdotn;
+  x.D = Ut[RHO];
+  double utsq = 0.;
+#pragma unroll
+  for (int i = 1; i < 4; i++)
+#pragma unroll
+    for (int j = 1; j < 4; j++) {
+      const double t = c[sym(i, j)] * pr[U1 + i - 1] * pr[U1 + j - 1];
+      utsq = (i == 1 && j == 1) ? t : utsq + t;
+    }
+  const double utsq_too_big = ((gammafail - 1.0) * (gammafail - 1.0));
+  ex.need(utsq >= 0. && utsq <= utsq_too_big);
+  const double p0 = (gam - 1.) * pr[UU], w0 = pr[RHO] + pr[UU] + p0;
+  x.wglobal = w0;
+  double W = w0 * (1. + utsq);
+  double x0 = fabs(W), ut = fabs(utsq_calc_x(ex, x, W));
+  double x1 = ex.Exact::div(ut, ex.rcp(ut + 1.));
+  const int ret = newton_vsq_x(ex, x, x0, x1, gammafail, *niter, maxit, nst, nss, resume);
+  if (ret == NEWTON_DEFERRED) return NEWTON_DEFERRED;
+#pragma unroll
+  for (int k = B1; k <= B3; k++) pr[k] = ex.div(Ut[k], ral);
+  if (ret != 0) return ret * 100 + 1;
+  W = x0;
+  if (W == FAIL_VAL) return 1;
+  if (Exact::quot(W, ex.rcp(w0)) > W_TOO_BIG) return PF_CONVW;
+  utsq = utsq_calc_x(ex, x, W);
+  if ((utsq < 0.) && (fabs(utsq) < 1.0e-13)) utsq = fabs(utsq);
+  if (utsq < 0. || utsq > utsq_too_big) return PF_CONVUTSQ2;
+  const double gamma = ex.sqrt_of(1. + utsq);
+  const double rho0 = ex.Exact::div(x.D, ex.rcp(gamma));
+  const double w = Exact::quot(W, ex.rcp(gamma * gamma));
+  const double p = ex.Exact::div((gam - 1.) * (w - rho0), ex.rcp(gam));
+  const double u = w - (rho0 + p);
+  int pfl = 0;
+  if ((rho0 <= 0.) || (u <= 0.)) {
+    if ((rho0 <= 0.) && (u >= 0.)) pfl = PF_RHONEG;
+    if ((rho0 >= 0.) && (u <= 0.)) pfl = PF_UNEG;
+    if ((rho0 <= 0.) && (u <= 0.)) pfl = PF_RHOUNEG;
+  }
+  pr[RHO] = rho0;
+  pr[UU] = u;
+  const double WB = W + x.Bsq;
+  const Recip r1 = ex.rcp(WB), r2 = ex.rcp(W * WB);
+#pragma unroll
+  for (int i = 1; i < 4; i++) {
+    const double Qt = Qcon[i] + (gn[i] * nlapse) * x.Qdotn;
+    const double t1 = ex.Exact::div(-gamma * Qt, r1), n2 = gamma * QdotB * B[i - 1];
+    // the field's part is watched only where the other does not drown it
+    ex.numerator((fabs(t1) > 1.e-150) ? 0. : n2);
+    pr[U1 + i - 1] = t1 - Exact::quot(n2, r2);
+  }
+  return pfl;
+}
+
+// utoprim_ffde and fixup1zone's Lorentz limit the same way
+__device__ __forceinline__ void utoprim_ffde_x(ExactTiny& ex, const double* U, const double* c, const double* gn,
+                                               double sg, double* pr, double gammamax)
+{
+  const Recip rs = ex.rcp(sg);
+  double S[3], B[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    S[k] = ex.div(U[U1 + k], rs);
+    B[k] = ex.div(U[B1 + k], rs);
+  }
+  const double alphasq = Exact::quot(1., ex.rcp(-gn[0]));
+  const double b1 = c[4] * B[0] + c[5] * B[1] + c[6] * B[2], b2 = c[5] * B[0] + c[7] * B[1] + c[8] * B[2];
+  const double b3 = c[6] * B[0] + c[8] * B[1] + c[9] * B[2];
+  const double Bsq = b1 * B[0] + b2 * B[1] + b3 * B[2];
+  const double o = Exact::quot(1., ex.rcp(Bsq * sg));
+  const double E1 = (b2 * S[2] - b3 * S[1]) * o, E2 = (b3 * S[0] - b1 * S[2]) * o, E3 = (b1 * S[1] - b2 * S[0]) * o;
+  const double e1 = c[4] * E1 + c[5] * E2 + c[6] * E3, e2 = c[5] * E1 + c[7] * E2 + c[8] * E3;
+  const double e3 = c[6] * E1 + c[8] * E2 + c[9] * E3;
+  const double Esq = E1 * e1 + E2 * e2 + E3 * e3;
+  const double gammasq = ex.Exact::div(Bsq, ex.rcp(Bsq - Esq));
+  ex.need(gammasq <= gammamax * gammamax && gammasq >= 1.0);
+  double v[4], uc[4];
+  v[1] = alphasq * (-gn[1] + (e2 * b3 - e3 * b2) * o);
+  v[2] = alphasq * (-gn[2] + (e3 * b1 - e1 * b3) * o);
+  v[3] = alphasq * (-gn[3] + (e1 * b2 - e2 * b1) * o);
+  const double discr = +c[0] + c[4] * v[1] * v[1] + c[7] * v[2] * v[2] + c[9] * v[3] * v[3] +
+                       2. * (c[1] * v[1] + c[2] * v[2] + c[3] * v[3] + c[5] * v[1] * v[2] + c[6] * v[1] * v[3] +
+                             c[8] * v[2] * v[3]);
+  uc[0] = Exact::quot(1., ex.rcp(ex.sqrt_of(-discr)));
+#pragma unroll
+  for (int j = 1; j < 4; j++) pr[U1 - 1 + j] = v[j] * uc[0];
+#pragma unroll
+  for (int k = 0; k < 3; k++) pr[B1 + k] = B[k];
+  const double qsq = c[4] * pr[U1] * pr[U1] + c[7] * pr[U2] * pr[U2] + c[9] * pr[U3] * pr[U3] +
+                     2. * (c[5] * pr[U1] * pr[U2] + c[6] * pr[U1] * pr[U3] + c[8] * pr[U2] * pr[U3]);
+  ex.need(gammamax <= 1.0 || ex.sqrt_of(1. + qsq) <= gammamax);
+}
+
+// flux divergence with flux-CT B fluxes (step_ch.c:1403-1413)
+template <typename FT>
+__device__ __forceinline__ void flux_divergence(const StepArgs& a, int i, int j, long long z, double* dUr)
+{
   const FT* F1 = reinterpret_cast<const FT*>(a.F1);
   const FT* F2 = reinterpret_cast<const FT*>(a.F2);
-  // block rows in launch order from both poles inward (0, last, 1, last-1,
-  // ...): the zones near the axis take the most Newton iterations, and
-  // started first their blocks no longer trail the kernel's last wave
-  // (developed 512^2 flow: 0.5256-0.5309 against 0.5333-0.5366 ms a step)
-  const unsigned by = (blockIdx.y & 1u) ? gridDim.y - 1u - (blockIdx.y >> 1) : (blockIdx.y >> 1);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = by * blockDim.y + threadIdx.y;
-  const int W = upd_box_w(blockDim.x);
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    mbar_init(&bar, 1);
-    mbar_expect_tx(&bar, (uint32_t)upd_smem_bytes(blockDim.x, blockDim.y));
-    tma_load_3d(sgeo, &geo_map, (int)((blockIdx.x * blockDim.x + NG) & ~1u), (int)(by * blockDim.y + NG),
-                GEO_CONN, &bar);
+  const long long pl = a.gr.plane;
+  const double idx1 = 1.0 / a.pp.dx1, idx2 = 1.0 / a.pp.dx2;
+  const long long zi1 = a.gr.at(i + 1, j), zj1 = a.gr.at(i, j + 1), zij = a.gr.at(i + 1, j + 1);
+  const double e00 = __ldg(a.emf + z), e10 = __ldg(a.emf + zi1), e01 = __ldg(a.emf + zj1), e11 = __ldg(a.emf + zij);
+#pragma unroll
+  for (int k = 0; k < NPR; k++) {
+    double f1p, f1m, f2p, f2m;
+    if (k == B1) {
+      f1p = 0.;
+      f1m = 0.;
+      f2m = -0.5 * (e00 + e10);
+      f2p = -0.5 * (e01 + e11);
+    } else if (k == B2) {
+      f1m = 0.5 * (e00 + e01);
+      f1p = 0.5 * (e10 + e11);
+      f2p = 0.;
+      f2m = 0.;
+    } else {
+      f1p = __ldg(F1 + k * pl + zi1);
+      f1m = __ldg(F1 + k * pl + z);
+      f2p = __ldg(F2 + k * pl + zj1);
+      f2m = __ldg(F2 + k * pl + z);
+    }
+    const double dU1 = (-(f1p - f1m) * idx1);
+    const double dU2 = (-(f2p - f2m) * idx2);
+    dUr[k] = dU1 + dU2;
   }
-  __syncthreads();  // the barrier is initialised before anyone polls it
-  const bool active = (i < a.gr.n1 && j < a.gr.n2);
-  const long long pl = a.gr.plane, z = a.gr.at(active ? i : 0, active ? j : 0);
-  const double dt = a.sc->dt;
+}
+
+// source_conn, phys.c:520-619: acc[l] = sum_j sum_k T^j_k Gamma^k_{lj}, T row
+// jj given, the connection planes in shared memory (sz, plane_s apart)
+__device__ __forceinline__ void source_row(const double* row, int jj, const double* sz, int plane_s, double* acc)
+{
+#pragma unroll
+  for (int l = 0; l < 4; l++)
+#pragma unroll
+    for (int k = 0; k < 4; k++) acc[l] += row[k] * sz[(conn_plane(k, l, jj) - GEO_CONN) * plane_s];
+}
+
+// a deferred (or, with the retry chain, failed) inversion goes to
+// k_update_tail, so that this warp is not held for up to 200 iterations by
+// one lane; -1 in the last state plane: to be solved afresh
+__device__ __forceinline__ void defer_zone(const StepArgs& a, long long z, int pfl, const double* U)
+{
+  const long long pl = a.gr.plane;
+  if (pfl != NEWTON_DEFERRED) a.fixbuf[(NEWTON_STATE - 1) * pl + z] = -1.0;
+#pragma unroll
+  for (int k = 0; k < NPR; k++) a.ubuf[k * pl + z] = U[k];
+  a.worklist[atomicAdd(&a.sc->ndeferred, 1)] = (int)z;
+}
+
+// one zone's update by the general templates; returns its Newton iterations
+template <typename FT, bool FFDE>
+__device__ __noinline__ int update_general(const StepArgs& a, int i, int j, const double* pi, const double* pb,
+                                           double* pf, double c2, const double* sz, int plane_s)
+{
+  const long long pl = a.gr.plane, z = a.gr.at(i, j);
+  const double dt = a.sc->dt, gam = a.pp.gam;
   Geo<double> g;
-  const double gam = a.pp.gam;
-  double U[NPR], pfz[NPR], dUr[NPR];
-  if (active) {
-    load_geo(a, CENT, z, g);
-    {
-      // Ui = U(pi)
-      double pr[NPR];
-#pragma unroll
-      for (int k = 0; k < NPR; k++) pr[k] = __ldg(pi + k * pl + z);
-#pragma unroll
-      for (int k = 0; k < NPR; k++) pfz[k] = pr[k];
-      State<double> q;
-      state_of(pr, g, q);
-      flux_of<double, FFDE>(pr, q, 0, g, gam, U);
-      if (a.bsqf_fused) a.bsqf_fused[z] = bsq_flag(a, pr, q);  // get_bsqflags of the step's p
-    }
-    {
-      // flux divergence with flux-CT B fluxes (step_ch.c:1403-1413)
-      const double idx1 = 1.0 / a.pp.dx1, idx2 = 1.0 / a.pp.dx2;
-      const long long zi1 = a.gr.at(i + 1, j), zj1 = a.gr.at(i, j + 1), zij = a.gr.at(i + 1, j + 1);
-      const double e00 = a.emf[z], e10 = a.emf[zi1], e01 = a.emf[zj1], e11 = a.emf[zij];
-#pragma unroll
-      for (int k = 0; k < NPR; k++) {
-        double f1p, f1m, f2p, f2m;
-        if (k == B1) {
-          f1p = 0.;
-          f1m = 0.;
-          f2m = -0.5 * (e00 + e10);
-          f2p = -0.5 * (e01 + e11);
-        } else if (k == B2) {
-          f1m = 0.5 * (e00 + e01);
-          f1p = 0.5 * (e10 + e11);
-          f2p = 0.;
-          f2m = 0.;
-        } else {
-          f1p = F1[k * pl + zi1];
-          f1m = F1[k * pl + z];
-          f2p = F2[k * pl + zj1];
-          f2m = F2[k * pl + z];
-        }
-        const double dU1 = (-(f1p - f1m) * idx1);
-        const double dU2 = (-(f2p - f2m) * idx2);
-        dUr[k] = dU1 + dU2;
-      }
-    }
-  }
-  if (!mbar_wait(&bar, 0)) {
-    if (active) report_fail(a.sc, a.phase0 + PH_UPDATE, FAIL_TMA_TIMEOUT, zone_order(i, j));
-    return;
-  }
-  if (!active) return;
-  const int plane_s = blockDim.y * W;
-  const double* sz = sgeo + threadIdx.y * W + threadIdx.x + 1;
-  double dUg[NPR];
+  load_geo(a, CENT, z, g);
+  double U[NPR], pfz[NPR], dUr[NPR], dUg[NPR];
   {
-    // source_conn, phys.c:520-619: dU[UU+l] = e * sum_j sum_k T^j_k Gamma^k_{lj}
+    // Ui = U(pi)
+    double pr[NPR];
+#pragma unroll
+    for (int k = 0; k < NPR; k++) pr[k] = __ldg(pi + k * pl + z);
+#pragma unroll
+    for (int k = 0; k < NPR; k++) pfz[k] = pr[k];
+    State<double> q;
+    state_of(pr, g, q);
+    flux_of<double, FFDE>(pr, q, 0, g, gam, U);
+    if (a.bsqf_fused) a.bsqf_fused[z] = bsq_flag(a, pr, q);  // get_bsqflags of the step's p
+  }
+  flux_divergence<FT>(a, i, j, z, dUr);
+  {
     double pr[NPR];
 #pragma unroll
     for (int k = 0; k < NPR; k++) pr[k] = __ldg(pb + k * pl + z);
@@ -902,10 +1140,7 @@ __global__ void __launch_bounds__(128, 4) k_update(StepArgs a, const __grid_cons
     for (int jj = 0; jj < 4; jj++) {
       double row[4];
       mhd_row<double, FFDE>(pr, jj, q, gam, row);
-#pragma unroll
-      for (int l = 0; l < 4; l++)
-#pragma unroll
-        for (int k = 0; k < 4; k++) acc[l] += row[k] * sz[(conn_plane(k, l, jj) - GEO_CONN) * plane_s];
+      source_row(row, jj, sz, plane_s, acc);
     }
     dUg[RHO] = 0. + g.g * 0.;
     dUg[B1] = dUg[B2] = dUg[B3] = dUg[RHO];
@@ -926,32 +1161,158 @@ __global__ void __launch_bounds__(128, 4) k_update(StepArgs a, const __grid_cons
     if (rc) report_fail(a.sc, a.phase0 + PH_UPDATE, rc, zone_order(i, j));
 #pragma unroll
     for (int k = 0; k < NPR; k++) pf[k * pl + z] = pfz[k];
-    return;
-  }
-  int niter;
-  // a deferred solve leaves its Newton state in the repair scratch (idle
-  // until k_fixup_compute), NEWTON_STATE planes
-  int pfl = utoprim_2d(U, g, pfz, gam, a.pp.gammafail, &niter, NEWTON_MAIN_CAP, a.fixbuf + z, pl);
-  if (pfl == NEWTON_DEFERRED || (a.pp.tryagain && pfl != 0)) {
-    // rare slow inversion: hand the zone to k_update_tail so that this warp
-    // is not held for up to 200 iterations by one lane (with the retry
-    // chain on, failed inversions go there too, to be solved afresh)
-    if (pfl != NEWTON_DEFERRED) a.fixbuf[(NEWTON_STATE - 1) * pl + z] = -1.0;
-#pragma unroll
-    for (int k = 0; k < NPR; k++) a.ubuf[k * pl + z] = U[k];
-    a.worklist[atomicAdd(&a.sc->ndeferred, 1)] = (int)z;
-    niter = 0;
+    return 0;
   } else {
+    int niter;
+    // a deferred solve leaves its Newton state in the repair scratch (idle
+    // until k_fixup_compute), NEWTON_STATE planes
+    const int pfl = utoprim_2d(U, g, pfz, gam, a.pp.gammafail, &niter, NEWTON_MAIN_CAP, a.fixbuf + z, pl);
+    if (pfl == NEWTON_DEFERRED || (a.pp.tryagain && pfl != 0)) {
+      defer_zone(a, z, pfl, U);
+      return 0;
+    }
     finish_zone(a, g, z, i, j, pfz, pfl, pf, sz[(GEO_FLOOR - GEO_CONN) * plane_s],
                 sz[(GEO_FLOOR + 1 - GEO_CONN) * plane_s]);
+    return niter;
   }
-  // Newton iteration count (the reference's nstroke), one atomic per warp
-  const unsigned mask = __activemask();
-  const unsigned it = __reduce_add_sync(mask, (unsigned)niter);
-  if ((int)(threadIdx.x & 31) == __ffs(mask) - 1) atomicAdd(&a.sc->newton_iters, (unsigned long long)it);
 }
 
-
+// advance_standard zone loop, advance.c:114-181, for one RK2 substep.
+// CUf = {1, 0, c2}: Uf = Ui + c2*dt*dU; on the last substep unew = Uf.
+// The connection coefficients and floors arrive by TMA (geo_map, a 3D map
+// over the geometry block with the box above) while U(p_i) is formed; the
+// block width is even.  Bound by memory latency, then by HBM (836 B a zone):
+// every global load starts before anything is computed, without branches in
+// between (harm_exact.cuh), at 168 registers (12 warps per SM; at 128 the
+// loads come in small batches and 172 B of registers spill: 66.6 against 61.5
+// us with the tail at 512^2).  A zone whose values leave the exact range goes
+// to update_general.  512^2 developed flow: 86 -> 50 us (first substep) and
+// 58 us (second), 3.9 TB/s; 1024^2 with the tail 300 -> 178 us.
+template <typename FT, bool FFDE>
+__global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepArgs a,
+                                                   const __grid_constant__ CUtensorMap geo_map,
+                                                   const double* __restrict__ pi, const double* __restrict__ pb,
+                                                   double* __restrict__ pf, double c2)
+{
+  extern __shared__ __align__(128) double sgeo[];
+  __shared__ uint64_t bar;
+  // block rows in launch order from both poles inward (0, last, 1, last-1,
+  // ...): the zones near the axis take the most Newton iterations, and
+  // started first their blocks no longer trail the kernel's last wave
+  // (developed 512^2 flow: 0.5256-0.5309 against 0.5333-0.5366 ms a step)
+  const unsigned by = (blockIdx.y & 1u) ? gridDim.y - 1u - (blockIdx.y >> 1) : (blockIdx.y >> 1);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = by * blockDim.y + threadIdx.y;
+  const int W = upd_box_w(blockDim.x);
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
+    mbar_init(&bar, 1);
+    mbar_expect_tx(&bar, (uint32_t)upd_smem_bytes(blockDim.x, blockDim.y));
+    tma_load_3d(sgeo, &geo_map, (int)((blockIdx.x * blockDim.x + NG) & ~1u), (int)(by * blockDim.y + NG),
+                GEO_CONN, &bar);
+  }
+  const bool active = (i < a.gr.n1 && j < a.gr.n2);
+  const long long pl = a.gr.plane, z = a.gr.at(active ? i : 0, active ? j : 0);
+  const double dt = a.sc->dt, gam = a.pp.gam;
+  double c[10], gn[10], sg;
+  double U[NPR], pfz[NPR], dUr[NPR];
+  ExactTiny ex;
+  StateX q;
+  LapseX lp;
+  unsigned char bf = 0;
+  // the flux divergence first, while few registers are taken: its 28 loads
+  // then start together (formed after U(pi), in small batches, they cost 20
+  // of the kernel's 79 us at 512^2)
+  flux_divergence<FT>(a, active ? i : 0, active ? j : 0, z, dUr);
+  {
+    const double* base = a.geo + (long long)CENT * GEO_PER_LOC * pl + z;
+#pragma unroll
+    for (int k = 0; k < 10; k++) c[k] = __ldg(base + k * pl);
+#pragma unroll
+    for (int k = 0; k < 10; k++) gn[k] = __ldg(base + (10 + k) * pl);
+    sg = __ldg(base + 20 * pl);
+#pragma unroll
+    for (int k = 0; k < NPR; k++) pfz[k] = __ldg(pi + k * pl + z);
+  }
+  // p_b is on its way meanwhile (asm: the compiler would load it at its use)
+  double prb[NPR];
+#pragma unroll
+  for (int k = 0; k < NPR; k++) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(prb[k]) : "l"(pb + k * pl + z));
+  __syncthreads();  // the barrier is initialised before anyone polls it
+  if (active) {
+    lp = lapse_x(ex, gn);
+    state_x(ex, pfz, c, lp, 1.e300, q);
+    // Ui = U(pi)
+    conserved_x<FFDE>(pfz, q, sg, gam, U);
+    if (a.bsqf_fused) bf = bsq_flag_x(ex, a, pfz, q.bsq);  // get_bsqflags of the step's p
+  }
+  if (!mbar_wait(&bar, 0)) {
+    if (active) report_fail(a.sc, a.phase0 + PH_UPDATE, FAIL_TMA_TIMEOUT, zone_order(i, j));
+    return;
+  }
+  if (!active) return;
+  const int plane_s = blockDim.y * W;
+  const double* sz = sgeo + threadIdx.y * W + threadIdx.x + 1;
+  {
+    // (the first substep's pb is pi, whose state is at hand)
+    if (pb != pi) state_x(ex, prb, c, lp, 1.e300, q);
+    const double r = FFDE ? 0. : prb[RHO], u = FFDE ? 0. : prb[UU], P = (gam - 1.) * u, w = P + r + u;
+    const double eta = FFDE ? q.bsq : w + q.bsq, ptot = FFDE ? q.bsq * 0.5 : P + q.bsq * 0.5;
+    double acc[4] = {0., 0., 0., 0.};
+#pragma unroll
+    for (int jj = 0; jj < 4; jj++) {
+      const double eu = eta * q.ucon[jj];
+      double row[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        double t = eu * q.ucov[k];
+        if (k == jj) t = t + ptot;
+        row[k] = t - q.bcon[jj] * q.bcov[k];
+      }
+      source_row(row, jj, sz, plane_s, acc);
+    }
+    // the RK combine of dUtoU, advance.c:273-286
+    const double cdt = c2 * dt;
+#pragma unroll
+    for (int k = 0; k < NPR; k++) {
+      const double d = (k >= UU && k <= U3) ? dUr[k] + sg * acc[k - UU] : dUr[k];
+      U[k] = U[k] + cdt * d;
+    }
+  }
+  if constexpr (FFDE) {
+    utoprim_ffde_x(ex, U, c, gn, sg, pfz, a.pp.gammamax);
+    if (!ex.ok()) {
+      update_general<FT, FFDE>(a, i, j, pi, pb, pf, c2, sz, plane_s);
+      return;
+    }
+#pragma unroll
+    for (int k = 0; k < NPR; k++) pf[k * pl + z] = pfz[k];
+  } else {
+    int niter;
+    // a deferred solve leaves its Newton state in the repair scratch (idle
+    // until k_fixup_compute), NEWTON_STATE planes
+    const int pfl = utoprim_2d_x(ex, U, c, gn, sg, pfz, gam, a.pp.gammafail, &niter, NEWTON_MAIN_CAP, a.fixbuf + z, pl,
+                                 false);
+    if (!ex.ok()) {
+      niter = update_general<FT, FFDE>(a, i, j, pi, pb, pf, c2, sz, plane_s);
+    } else {
+      if (a.bsqf_fused) a.bsqf_fused[z] = bf;
+      if (pfl == NEWTON_DEFERRED || (a.pp.tryagain && pfl != 0)) {
+        defer_zone(a, z, pfl, U);
+        niter = 0;
+      } else {
+        Geo<double> g;
+#pragma unroll
+        for (int k = 0; k < 10; k++) g.gcov[k] = c[k];
+        finish_zone(a, g, z, i, j, pfz, pfl, pf, sz[(GEO_FLOOR - GEO_CONN) * plane_s],
+                    sz[(GEO_FLOOR + 1 - GEO_CONN) * plane_s]);
+      }
+    }
+    // Newton iteration count (the reference's nstroke), one atomic per warp
+    const unsigned mask = __activemask();
+    const unsigned it = __reduce_add_sync(mask, (unsigned)niter);
+    if ((int)(threadIdx.x & 31) == __ffs(mask) - 1) atomicAdd(&a.sc->newton_iters, (unsigned long long)it);
+  }
+}
 
 // launches a k_update instance (its dynamic shared memory limit raised once
 // to the largest box of the tile shapes harm_set_tiles accepts: 42 planes x
