@@ -79,37 +79,115 @@ __device__ __forceinline__ int utoprim_2d_full(const double* U, const Geo<double
 // The deferred inversions of k_update, continued from the Newton state
 // k_update saved (repair scratch planes 0-4) up to the full iteration limit.
 // A deferred zone's pf slot was not written, so pi still holds its guess.
-// TA: the UTOPRIMTRYAGAIN retry chain follows a failed 2D inversion (those
-// zones carry no saved state and are solved afresh).
-template <bool TA>
+// (With the retry chain, failed inversions come here too: they carry no
+// saved state and are solved afresh.)
+__device__ __forceinline__ int tail_2d(const StepArgs& a, const double* __restrict__ pi, long long z,
+                                       const Geo<double>& g, double* U, double* pfz, int* niter)
+{
+  const long long pl = a.gr.plane;
+#pragma unroll
+  for (int k = 0; k < NPR; k++) {
+    U[k] = a.ubuf[k * pl + z];
+    pfz[k] = pi[k * pl + z];
+  }
+  double* nst = a.fixbuf + z;
+  const bool resume = nst[(NEWTON_STATE - 1) * pl] >= 0.0;
+  return utoprim_2d_full(U, g, pfz, a.pp.gam, a.pp.gammafail, niter, nst, pl, resume);
+}
+__device__ __forceinline__ void tail_finish(const StepArgs& a, const Geo<double>& g, long long z, double* pfz, int pfl,
+                                            double* pf)
+{
+  finish_zone(a, g, z, (int)(z % a.gr.pitch) - NG, (int)(z / a.gr.pitch) - NG, pfz, pfl, pf,
+              __ldg(a.geo + (long long)GEO_FLOOR * a.gr.plane + z),
+              __ldg(a.geo + (long long)(GEO_FLOOR + 1) * a.gr.plane + z));
+}
+
 __global__ void __launch_bounds__(64) k_update_tail(StepArgs a, const double* __restrict__ pi, double* __restrict__ pf)
 {
   const int nd = a.sc->ndeferred;
-  const long long pl = a.gr.plane;
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < nd; w += gridDim.x * blockDim.x) {
     const long long z = a.worklist[w];
-    const int i = (int)(z % a.gr.pitch) - NG, j = (int)(z / a.gr.pitch) - NG;
     Geo<double> g;
     load_geo(a, CENT, z, g);
     double U[NPR], pfz[NPR];
-#pragma unroll
-    for (int k = 0; k < NPR; k++) {
-      U[k] = a.ubuf[k * pl + z];
-      pfz[k] = pi[k * pl + z];
-    }
     int niter;
-    double* nst = a.fixbuf + z;
-    const bool resume = nst[(NEWTON_STATE - 1) * pl] >= 0.0;
-    int pfl = utoprim_2d_full(U, g, pfz, a.pp.gam, a.pp.gammafail, &niter, nst, pl, resume);
-    if (TA && pfl != 0) {
-      double pr0[NPR];
-#pragma unroll
-      for (int k = 0; k < NPR; k++) pr0[k] = pi[k * pl + z];
-      pfl = ta::tryagain_chain(U, g, a.pp.gam, a.pp.gammafail, pr0, pfz, pfl);
-    }
-    finish_zone(a, g, z, i, j, pfz, pfl, pf, __ldg(a.geo + (long long)GEO_FLOOR * pl + z),
-                __ldg(a.geo + (long long)(GEO_FLOOR + 1) * pl + z));
+    const int pfl = tail_2d(a, pi, z, g, U, pfz, &niter);
+    tail_finish(a, g, z, pfz, pfl, pf);
     atomicAdd(&a.sc->newton_iters, (unsigned long long)niter);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.sc->ndeferred_total += nd;
+}
+
+// The same with the UTOPRIMTRYAGAIN retry chain after a failed 2D inversion
+// (ta::tryagain_chain).  A handful of zones fail a substep, and one that
+// fails every method took its 2.2 ms one after another (0.56 5D1, 0.6 1D,
+// 0.55 1D_OPT, 0.32 and 0.13 the final 1D and 2D, 1.06 5D2; everything else
+// waits).  Here a block's warps run its zones' methods side by side; the
+// first in the chain's order that succeeds is the result, and the methods
+// after it stop.  The worklist is dealt out over the blocks zone by zone, so
+// that lanes of a warp rarely share a solve's branches.  245 x 131 torus, a
+// few failures a substep: the update and its tail 1.92 -> 1.57 ms a substep;
+// what is left is the dependency chain of the slowest method (5D2, 5.7 us an
+// iteration) and instruction fetch (six methods' code on one SM).
+constexpr int TAIL_CHAIN = 6;  // methods after the primary 2D (the chain's own 2D repeats it)
+__global__ void __launch_bounds__(32 * TAIL_CHAIN) k_update_tail_chain(StepArgs a, const double* __restrict__ pi,
+                                                                      double* __restrict__ pf)
+{
+  __shared__ double res[TAIL_CHAIN][NPR][32];
+  __shared__ int code[TAIL_CHAIN][32], won[32], list[32 * TAIL_CHAIN], nlist;
+  const int nd = a.sc->ndeferred, lane = threadIdx.x & 31, m = threadIdx.x >> 5;
+  const long long pl = a.gr.plane;
+  const int order[TAIL_CHAIN] = {ta::M_5D1, ta::M_1D, ta::M_1DOPT, ta::M_1DFINAL, ta::M_2DFINAL, ta::M_5D2};
+  for (int first = blockIdx.x; first < nd; first += gridDim.x * blockDim.x) {
+    if (threadIdx.x == 0) nlist = 0;
+    __syncthreads();
+    const int w = first + gridDim.x * threadIdx.x;
+    if (w < nd) {
+      const long long z = a.worklist[w];
+      Geo<double> g;
+      load_geo(a, CENT, z, g);
+      double U[NPR], pfz[NPR];
+      int niter;
+      const int pfl = tail_2d(a, pi, z, g, U, pfz, &niter);
+      if (pfl == 0) tail_finish(a, g, z, pfz, pfl, pf);
+      else list[atomicAdd(&nlist, 1)] = (int)z;
+      atomicAdd(&a.sc->newton_iters, (unsigned long long)niter);
+    }
+    __syncthreads();
+    for (int c0 = 0; c0 < nlist; c0 += 32) {
+      const bool act = c0 + lane < nlist;
+      const long long z = act ? list[c0 + lane] : 0;
+      if (m == 0) won[lane] = TAIL_CHAIN;
+      __syncthreads();
+      if (act) {
+        Geo<double> g;
+        load_geo(a, CENT, z, g);
+        double U[NPR], Ug[NPR], p[NPR];
+#pragma unroll
+        for (int k = 0; k < NPR; k++) {
+          U[k] = a.ubuf[k * pl + z];
+          p[k] = pi[k * pl + z];
+        }
+        ta::evolved_to_geomfree(U, g, Ug);
+        const int f = ta::pick(order[m], Ug, g, a.pp.gam, a.pp.gammafail, p, ta::Stop{&won[lane], m});
+#pragma unroll
+        for (int k = 0; k < NPR; k++) res[m][k][lane] = p[k];
+        code[m][lane] = f;
+        if (f == 0) atomicMin(&won[lane], m);
+      }
+      __syncthreads();
+      if (m == 0 && act) {
+        // the chain's result: the first success, or the last method's
+        const int b = (won[lane] < TAIL_CHAIN) ? won[lane] : TAIL_CHAIN - 1;
+        Geo<double> g;
+        load_geo(a, CENT, z, g);
+        double pfz[NPR];
+#pragma unroll
+        for (int k = 0; k < NPR; k++) pfz[k] = res[b][k][lane];
+        tail_finish(a, g, z, pfz, code[b][lane], pf);
+      }
+      __syncthreads();
+    }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) a.sc->ndeferred_total += nd;
 }
@@ -961,8 +1039,8 @@ void launch_update(int mixed, int ffde, dim3 g, dim3 b, cudaStream_t s, const St
   else if (ffde) update_launch<double, true>(g, b, s, a, map, pi, pb, pf, c2);
   else update_launch<double, false>(g, b, s, a, map, pi, pb, pf, c2);
   if (!ffde) {
-    if (a.pp.tryagain) k_update_tail<true><<<148, 64, 0, s>>>(a, pi, pf);
-    else k_update_tail<false><<<148, 64, 0, s>>>(a, pi, pf);
+    if (a.pp.tryagain) k_update_tail_chain<<<148, 32 * TAIL_CHAIN, 0, s>>>(a, pi, pf);
+    else k_update_tail<<<148, 64, 0, s>>>(a, pi, pf);
   }
 }
 

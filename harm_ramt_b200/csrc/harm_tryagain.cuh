@@ -5,7 +5,8 @@
 //   5D1 (utoprim.c + mnewt.c + dudp_calc.c), 2D again, 1D, 1D_OPT,
 //   1D_FINAL, 2D_FINAL, 5D2_FINAL.
 // A cold path: the chain runs only on the zones whose 2D inversion failed
-// (a compacted list), one thread per zone.  Every method is restated with
+// (a compacted list); k_update_tail_chain runs a zone's methods side by side,
+// a warp each.  Every method is restated with
 // the reference's evaluation order so that the chain's result is the
 // reference's bit for bit.  Host-and-device, so that the same code can be
 // compared with the reference build on the CPU.
@@ -20,6 +21,14 @@ namespace ta {
 // method ids of Utoprimgen_pick, step_ch.h:39-53
 enum { M_5D1 = 0, M_LDZ = 1, M_2D = 2, M_1D = 3, M_1DOPT = 4, M_1DFINAL = 5, M_2DFINAL = 6, M_5D2 = 7 };
 constexpr int PF_CONV = 1;  // UTOPRIMFAILCONV, global.h:550
+
+// Where the methods of a zone's chain run side by side: a method whose place
+// is after one that has succeeded ends (its result is not looked at)
+struct Stop {
+  const volatile int* won = nullptr;  // the first place that has succeeded so far
+  int place = 0;
+  HD_INLINE bool operator()() const { return won && *won < place; }
+};
 
 HD_INLINE double gcov_at(const Geo<double>& g, int j, int k) { return g.gcov[sym(j, k)]; }
 HD_INLINE double kdelta(int a, int b) { return (a == b) ? 1.0 : 0.0; }
@@ -143,31 +152,37 @@ HD_INLINE void usrfun5(const double* pr, const Geo<double>& g, double gam, const
 // here).  A singular row leaves the decomposition unfinished as the
 // reference's early return does; the pivots of unfinished columns are then
 // the identity (the reference reuses stale static state there).
+// (All indices are constants after unrolling -- a pivot row is picked by
+// comparing -- so that the matrix stays in registers.)
 HD_INLINE void lu_solve5(double a[5][5], double b[5], int indx[5])
 {
   double vv[5];
   int singular = 0;
+#pragma unroll
   for (int i = 0; i < 5; i++) {
     double big = 0.0, temp;
+#pragma unroll
     for (int j = 0; j < 5; j++)
       if ((temp = fabs(a[i][j])) > big) big = temp;
-    if (big == 0.0) {
-      singular = 1;
-      break;
-    }
+    if (big == 0.0) singular = 1;
     vv[i] = 1.0 / big;
   }
   if (!singular) {
+#pragma unroll
     for (int j = 0; j < 5; j++) {
       int imax = -1;
+#pragma unroll
       for (int i = 0; i < j; i++) {
         double sum = a[i][j];
+#pragma unroll
         for (int k = 0; k < i; k++) sum -= a[i][k] * a[k][j];
         a[i][j] = sum;
       }
       double big = 0.0, dum;
+#pragma unroll
       for (int i = j; i < 5; i++) {
         double sum = a[i][j];
+#pragma unroll
         for (int k = 0; k < j; k++) sum -= a[i][k] * a[k][j];
         a[i][j] = sum;
         if ((dum = vv[i] * fabs(sum)) >= big) {
@@ -176,35 +191,49 @@ HD_INLINE void lu_solve5(double a[5][5], double b[5], int indx[5])
         }
       }
       if (imax < 0) imax = j;  // a NaN column: no pivot found
-      if (j != imax) {
-        for (int k = 0; k < 5; k++) {
-          dum = a[imax][k];
-          a[imax][k] = a[j][k];
-          a[j][k] = dum;
+#pragma unroll
+      for (int r = j + 1; r < 5; r++)
+        if (r == imax) {
+#pragma unroll
+          for (int k = 0; k < 5; k++) {
+            dum = a[r][k];
+            a[r][k] = a[j][k];
+            a[j][k] = dum;
+          }
+          vv[r] = vv[j];
         }
-        vv[imax] = vv[j];
-      }
       indx[j] = imax;
       if (a[j][j] == 0.0) a[j][j] = 1.0e-30;
       if (j != 4) {
         dum = 1.0 / (a[j][j]);
+#pragma unroll
         for (int i = j + 1; i < 5; i++) a[i][j] *= dum;
       }
     }
   }
   int ii = -1;
+#pragma unroll
   for (int i = 0; i < 5; i++) {
     const int ip = indx[i];
-    double sum = b[ip];
-    b[ip] = b[i];
-    if (ii >= 0)
-      for (int j = ii; j <= i - 1; j++) sum -= a[i][j] * b[j];
-    else if (sum != 0.0)
+    double sum = b[i];
+#pragma unroll
+    for (int r = 0; r < 5; r++)
+      if (r == ip) {
+        sum = b[r];
+        b[r] = b[i];
+      }
+    if (ii >= 0) {
+#pragma unroll
+      for (int j = 0; j < i; j++)
+        if (j >= ii) sum -= a[i][j] * b[j];
+    } else if (sum != 0.0)
       ii = i;
     b[i] = sum;
   }
+#pragma unroll
   for (int i = 4; i >= 0; i--) {
     double sum = b[i];
+#pragma unroll
     for (int j = i + 1; j < 5; j++) sum -= a[i][j] * b[j];
     b[i] = sum / a[i][i];
   }
@@ -214,7 +243,7 @@ HD_INLINE void lu_solve5(double a[5][5], double b[5], int indx[5])
 // startp = RHO): damped Newton on x = pr[0..4].  Returns 0 when converged
 // (or within the allowed tolerances), 1 otherwise.
 HD_INLINE int mnewt5(int ntrial, int mintrial, double* x, const Geo<double>& g, double gam, const double* Utarget,
-                     double tolx, double tolf, double tolxallowed, double tolfallowed)
+                     double tolx, double tolf, double tolxallowed, double tolfallowed, Stop stop)
 {
   const double abstol = DBL_EPS_REF * 50.0, abstolhard = DBL_EPS_REF;
   if (tolx < abstol) tolx = abstol;
@@ -229,6 +258,7 @@ HD_INLINE int mnewt5(int ntrial, int mintrial, double* x, const Geo<double>& g, 
   double xold[5], fvec[5], fjac[5][5], pp[5], pptest[5], normf;
   for (int i = 0; i < 5; i++) xold[i] = x[i];
   for (int k = 1; k <= ntrial; k++) {
+    if (stop()) return 1;
     usrfun5(x, g, gam, Utarget, fvec, fjac, &normf);
     errf = 0.0;
     for (int i = 0; i < 5; i++) errf += fabs(fvec[i]);
@@ -314,7 +344,7 @@ HD_INLINE int mnewt5(int ntrial, int mintrial, double* x, const Geo<double>& g, 
 // Utoprim (5D1), utoprim.c:24-318 with EVOLVENOENTROPY, PRECISEINVERSION 1
 // and nutoprims = 1.  Ug: geometry-free U (UNOTHING); pr: guess in, result
 // out.  Returns the pflag code.
-HD_INLINE int utoprim_5d1(const double* Ug, const Geo<double>& g, double gam, double* pr)
+HD_INLINE int utoprim_5d1(const double* Ug, const Geo<double>& g, double gam, double* pr, Stop stop)
 {
   for (int k = B1; k <= B3; k++) pr[k] = Ug[k];
   double pr0[NPR], priter[NPR], Utarget[NPR], Ustart[NPR], dU[NPR];
@@ -330,7 +360,7 @@ HD_INLINE int utoprim_5d1(const double* Ug, const Geo<double>& g, double gam, do
   const int countutoprims = 1;
   const double frac = 1.0 / ((double)1);
   for (int k = 0; k < NPR; k++) Utarget[k] = Ustart[k] + dU[k] * (double)countutoprims * frac;
-  const int failed = mnewt5(200, 3, priter, g, gam, Utarget, 1.e-11, 1.e-11, 1.e-8, 1.e-8);
+  const int failed = mnewt5(200, 3, priter, g, gam, Utarget, 1.e-11, 1.e-11, 1.e-8, 1.e-8, stop);
   for (int k = 0; k < NPR; k++) pr[k] = priter[k];
   if (failed) {
     for (int k = 0; k < NPR; k++) pr[k] = pr0[k];
@@ -353,6 +383,7 @@ HD_INLINE int utoprim_5d1(const double* Ug, const Geo<double>& g, double gam, do
 struct Noble {
   double Bsq, QdotBsq, Qtsq, Qdotn, D, wglobal, gam, gammafail;
   double QdotB, Bcon[4], Qcon[4], ncon[4];
+  Stop stop;
 };
 
 constexpr double N_W_TOO_BIG = 1.e9, N_FAIL_VAL = 1.e30, N_MAXNEGUTSQ = 1E-10;
@@ -491,6 +522,7 @@ HD_INLINE void n1_lnsrch(const Noble& c, double xold, double fold, double g, dou
   alamin = TOLX / test;
   alam = 1.0;
   for (int it = 0; it < N_LNSRCH_MAX; it++) {
+    if (c.stop()) break;
     x = xold + alam * p;
     f = n1_res_sq(c, x);
     const int bad_step = FINAL ? (isfinite(f) == 0) : (x <= 0.);
@@ -543,6 +575,7 @@ HD_INLINE int n1_gnr(const Noble& c, double& x)
   x_old = x_orig = x;
   bool keep_iterating = true;
   while (keep_iterating) {
+    if (c.stop()) return 1;
     n1_func(c, x, dx, resid, jac, f, df);
     if (n_iter == 0) {
       resid_norm = 0.0e0;
@@ -612,7 +645,8 @@ HD_INLINE int n1_gnr(const Noble& c, double& x)
 // Utoprim_1d / Utoprim_1d_opt with their Utoprim_new_body (utoprim_1d.c:19-321,
 // utoprim_1d_opt.c:19-375).  Ug: geometry-free U; prim: guess in, result out.
 template <bool OPT>
-HD_INLINE int utoprim_1d_family(const double* Ug, const Geo<double>& g, double gam, double gammafail, double* prim)
+HD_INLINE int utoprim_1d_family(const double* Ug, const Geo<double>& g, double gam, double gammafail, double* prim,
+                               Stop stop)
 {
   const double alpha = 1.0 / sqrt(-g.gcon[0]);
   double U[NPR], pr[NPR];
@@ -627,6 +661,7 @@ HD_INLINE int utoprim_1d_family(const double* Ug, const Geo<double>& g, double g
     for (int i = B1; i <= B3; i++) pr[i] = U[i];
     Noble c;
     noble_setup(U, g, gam, gammafail, c);
+    c.stop = stop;
     const double utsq_too_big = (gammafail - 1.0) * (gammafail - 1.0);
     double utsq = guess_utsq(pr, g);
     if (!OPT) {
@@ -758,6 +793,7 @@ HD_INLINE int nf1_gnr(const Noble& c, double& x)
   int n_iter = 0, i_extra = 0, doing_extra = 0;
   bool keep_iterating = true;
   while (keep_iterating) {
+    if (c.stop()) return 1;
     nf1_func(c, x, dx, f, df);
     errx = 0.;
     x += dx;
@@ -820,6 +856,7 @@ HD_INLINE int nf2_gnr(const Noble& c, double* x)
   int n_iter = 0, i_extra = 0, doing_extra = 0;
   bool keep_iterating = true;
   while (keep_iterating) {
+    if (c.stop()) return 1;
     nf2_func(c, x, dx, f, df);
     errx = 0.;
     x_old[0] = x[0];
@@ -847,7 +884,8 @@ HD_INLINE int nf2_gnr(const Noble& c, double* x)
 // Utoprim_1d_final / Utoprim_2d_final with their Utoprim_new_body
 // (utoprim_1d_final.c:26-397, utoprim_2d_final.c:26-397)
 template <bool TWO_D>
-HD_INLINE int utoprim_final_family(const double* Ug, const Geo<double>& g, double gam, double gammafail, double* prim)
+HD_INLINE int utoprim_final_family(const double* Ug, const Geo<double>& g, double gam, double gammafail, double* prim,
+                               Stop stop)
 {
   for (int i = B1; i <= B3; i++) prim[i] = Ug[i];
   const double alpha = 1.0 / sqrt(-g.gcon[0]);
@@ -860,6 +898,7 @@ HD_INLINE int utoprim_final_family(const double* Ug, const Geo<double>& g, doubl
     for (int i = B1; i <= B3; i++) pr[i] = U[i];
     Noble c;
     noble_setup(U, g, gam, gammafail, c);
+    c.stop = stop;
     double utsq = guess_utsq(pr, g);
     if ((utsq < 0.) && (fabs(utsq) < N_MAXNEGUTSQ)) utsq = 0.0;
     if (utsq < 0. || utsq > (gammafail - 1.0) * (gammafail - 1.0)) {
@@ -1009,27 +1048,31 @@ HD_INLINE void lu5_solve(double A[5][5], double* B)
 {
   int permute[5] = {0, 0, 0, 0, 0};
   double row_norm[5];
-  const int n = 5;
+  constexpr int n = 5;
   bool singular = false;
+#pragma unroll
   for (int i = 0; i < n; i++) {
     double absmax = 0.;
+#pragma unroll
     for (int j = 0; j < n; j++) {
       const double maxtemp = fabs(A[i][j]);
       if (maxtemp > absmax) absmax = maxtemp;
     }
-    if (absmax == 0.) {
-      singular = true;
-      break;
-    }
+    if (absmax == 0.) singular = true;
     row_norm[i] = 1. / absmax;
   }
   if (!singular) {
     int max_row = 0;
+#pragma unroll
     for (int j = 0; j < n; j++) {
+#pragma unroll
       for (int i = 0; i < j; i++)
+#pragma unroll
         for (int k = 0; k < i; k++) A[i][j] -= A[i][k] * A[k][j];
       double absmax = 0.0;
+#pragma unroll
       for (int i = j; i < n; i++) {
+#pragma unroll
         for (int k = 0; k < j; k++) A[i][j] -= A[i][k] * A[k][j];
         const double maxtemp = fabs(A[i][j]) * row_norm[i];
         if (maxtemp >= absmax) {
@@ -1037,33 +1080,49 @@ HD_INLINE void lu5_solve(double A[5][5], double* B)
           max_row = i;
         }
       }
+      // (a NaN column leaves max_row at an earlier column's row)
       if (max_row != j) {
-        if ((j == (n - 2)) && (A[j][j + 1] == 0.)) {
+        if ((j == (n - 2)) && (A[j][(j + 1 < n) ? j + 1 : j] == 0.)) {
           max_row = j;
         } else {
-          for (int k = 0; k < n; k++) {
-            const double t = A[j][k];
-            A[j][k] = A[max_row][k];
-            A[max_row][k] = t;
-          }
-          row_norm[max_row] = row_norm[j];
+#pragma unroll
+          for (int r = 0; r < n; r++)
+            if (r == max_row && r != j) {
+#pragma unroll
+              for (int k = 0; k < n; k++) {
+                const double t = A[j][k];
+                A[j][k] = A[r][k];
+                A[r][k] = t;
+              }
+              row_norm[r] = row_norm[j];
+            }
         }
       }
       permute[j] = max_row;
       if (A[j][j] == 0.) A[j][j] = 1e-30;
       if (j != (n - 1)) {
         const double maxtemp = 1. / A[j][j];
+#pragma unroll
         for (int i = (j + 1); i < n; i++) A[i][j] *= maxtemp;
       }
     }
   }
+#pragma unroll
   for (int i = 0; i < n; i++) {
-    double tmpvar = B[permute[i]];
-    B[permute[i]] = B[i];
+    double tmpvar = B[i];
+#pragma unroll
+    for (int r = 0; r < n; r++)
+      if (r == permute[i]) {
+        tmpvar = B[r];
+        B[r] = B[i];
+      }
+#pragma unroll
     for (int j = (i - 1); j >= 0; j--) tmpvar -= A[i][j] * B[j];
     B[i] = tmpvar;
   }
+#pragma unroll
   for (int i = (n - 1); i >= 0; i--) {
+#pragma unroll
     for (int j = (i + 1); j < n; j++) B[i] -= A[i][j] * B[j];
     B[i] /= A[i][i];
   }
@@ -1106,7 +1165,7 @@ HD_INLINE void f5d2_func(const double* x, const double* Utarget, const Geo<doubl
 // Utoprim_5d2_final with its general_newton_raphson (USE_LINE_SEARCH -2,
 // NEWCONVERGE 1, errx from W of calc_errx_5d), utoprim_5d2_final.c:28-75,
 // 352-372, 980-1300
-HD_INLINE int utoprim_5d2(const double* Ug, const Geo<double>& g, double gam, double* prim)
+HD_INLINE int utoprim_5d2(const double* Ug, const Geo<double>& g, double gam, double* prim, Stop stop)
 {
   constexpr double TOL_RESID = 1.e-4;
   double Utarget[NPR], x[NPR];
@@ -1119,6 +1178,7 @@ HD_INLINE int utoprim_5d2(const double* Ug, const Geo<double>& g, double gam, do
     int n_iter = 0, i_extra = 0, doing_extra = 0;
     bool keep_iterating = true;
     while (keep_iterating) {
+      if (stop()) return PF_CONV;
       f5d2_func(x, Utarget, g, gam, dx, f, df);
       errx = 0.;
       for (int id = 0; id < 5; id++) x[id] += dx[id];
@@ -1164,15 +1224,16 @@ HD_INLINE void evolved_to_geomfree(const double* U, const Geo<double>& g, double
 // Ug geometry-free, pr the guess in and the result out; returns the pflag
 // code.  The LDZ method is not part of the chain (step_ch.c:616 leaves it
 // out) and returns UTOPRIMFAILCONV here.
-HD_INLINE int pick(int which, const double* Ug, const Geo<double>& g, double gam, double gammafail, double* pr)
+HD_INLINE int pick(int which, const double* Ug, const Geo<double>& g, double gam, double gammafail, double* pr,
+                   Stop stop = Stop())
 {
   switch (which) {
-    case M_5D1: return utoprim_5d1(Ug, g, gam, pr);
-    case M_1D: return utoprim_1d_family<false>(Ug, g, gam, gammafail, pr);
-    case M_1DOPT: return utoprim_1d_family<true>(Ug, g, gam, gammafail, pr);
-    case M_1DFINAL: return utoprim_final_family<false>(Ug, g, gam, gammafail, pr);
-    case M_2DFINAL: return utoprim_final_family<true>(Ug, g, gam, gammafail, pr);
-    case M_5D2: return utoprim_5d2(Ug, g, gam, pr);
+    case M_5D1: return utoprim_5d1(Ug, g, gam, pr, stop);
+    case M_1D: return utoprim_1d_family<false>(Ug, g, gam, gammafail, pr, stop);
+    case M_1DOPT: return utoprim_1d_family<true>(Ug, g, gam, gammafail, pr, stop);
+    case M_1DFINAL: return utoprim_final_family<false>(Ug, g, gam, gammafail, pr, stop);
+    case M_2DFINAL: return utoprim_final_family<true>(Ug, g, gam, gammafail, pr, stop);
+    case M_5D2: return utoprim_5d2(Ug, g, gam, pr, stop);
     default: return PF_CONV;
   }
 }
