@@ -590,28 +590,26 @@ int harm_invert_zones(harm_ctx* c, int which, int nz, const int* zones, const do
     if (zones[2 * k] < 0 || zones[2 * k] >= c->cfg.n1 || zones[2 * k + 1] < 0 || zones[2 * k + 1] >= c->cfg.n2)
       return HARM_EINVAL;
   if (nz == 0) return HARM_OK;
-  int* dz = nullptr;
-  double *dU = nullptr, *dp = nullptr;
-  int* df = nullptr;
+  // one allocation: U, pr, the zones, the flags
+  double* dU = nullptr;
   int rc = HARM_OK;
   const size_t nd = (size_t)NPR * nz * sizeof(double);
-  if (cudaMalloc(&dz, 2 * nz * sizeof(int)) != cudaSuccess || cudaMalloc(&dU, nd) != cudaSuccess ||
-      cudaMalloc(&dp, nd) != cudaSuccess || cudaMalloc(&df, nz * sizeof(int)) != cudaSuccess)
-    rc = HARM_ENOMEM;
-  cudaStream_t s = c->stream;
-  if (rc == HARM_OK) {
-    cudaMemcpyAsync(dz, zones, 2 * nz * sizeof(int), cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(dU, U, nd, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(dp, pr, nd, cudaMemcpyHostToDevice, s);
-    k_invert_zones<<<(nz + 63) / 64, 64, 0, s>>>(c->args(), which, nz, dz, dU, dp, df);
-    cudaMemcpyAsync(pr, dp, nd, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(pflag, df, nz * sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = HARM_ECUDA;
+  if (cudaMalloc(&dU, 2 * nd + 3 * (size_t)nz * sizeof(int)) != cudaSuccess) {
+    cudaGetLastError();
+    return HARM_ENOMEM;
   }
-  cudaFree(dz);
+  double* dp = dU + (size_t)NPR * nz;
+  int* dz = (int*)(dp + (size_t)NPR * nz);
+  int* df = dz + 2 * (size_t)nz;
+  cudaStream_t s = c->stream;
+  cudaMemcpyAsync(dz, zones, 2 * (size_t)nz * sizeof(int), cudaMemcpyHostToDevice, s);
+  cudaMemcpyAsync(dU, U, nd, cudaMemcpyHostToDevice, s);
+  cudaMemcpyAsync(dp, pr, nd, cudaMemcpyHostToDevice, s);
+  k_invert_zones<<<(nz + 63) / 64, 64, 0, s>>>(c->args(), which, nz, dz, dU, dp, df);
+  cudaMemcpyAsync(pr, dp, nd, cudaMemcpyDeviceToHost, s);
+  cudaMemcpyAsync(pflag, df, nz * sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = HARM_ECUDA;
   cudaFree(dU);
-  cudaFree(dp);
-  cudaFree(df);
   return rc;
 }
 
@@ -978,23 +976,34 @@ namespace {
 // checkpoint segment runs from one set (on its own stream), the replay of
 // the segment before it records into the other (on the context's stream).
 struct AdjWork {
-  std::vector<void*> mem;
   std::vector<Rec> rec[2];        // one per step of a checkpoint segment, per set
   std::vector<double*> pnext[2];  // the state after each slot's step (the next slot's pn; an extra one at the end)
   std::vector<cudaGraphExec_t> recg[2];  // the recording step of each slot, captured
   std::vector<cudaGraphExec_t> adjg[2];  // the adjoint step of each slot, captured
   double *La, *Lc, *Lb, *Lsnap, *LdU, *Le, *Sr, *dts, *dot;
   DevScalars* sc_adj;  // the adjoint stream's scalars (its steps' dt), apart from the replay's
-  bool ok = true;
+  // one allocation holds everything: `plan` lays the pieces out twice, first
+  // to add up their sizes (get() then returns null), then to place them
+  // (some 500 allocations and their release took 0.15 s of a 0.28 s call)
+  char* base = nullptr;
+  size_t used = 0;
   void* get(size_t bytes)
   {
-    void* p = nullptr;
-    if (cudaMalloc(&p, bytes) != cudaSuccess) {
-      ok = false;
-      return nullptr;
-    }
-    mem.push_back(p);
+    void* p = base ? base + used : nullptr;
+    used += (bytes + 255) / 256 * 256;
     return p;
+  }
+  int alloc(const std::function<void()>& plan)
+  {
+    plan();
+    if (cudaMalloc(&base, used) != cudaSuccess) {
+      cudaGetLastError();
+      base = nullptr;
+      return HARM_ENOMEM;
+    }
+    used = 0;
+    plan();
+    return HARM_OK;
   }
   ~AdjWork()
   {
@@ -1004,7 +1013,7 @@ struct AdjWork {
       for (cudaGraphExec_t g : adjg[x])
         if (g) cudaGraphExecDestroy(g);
     }
-    for (void* p : mem) cudaFree(p);
+    cudaFree(base);
   }
 };
 
@@ -1025,7 +1034,7 @@ size_t dot_blocks(const harm_ctx* c)
 // 10 state-sized arrays, in each of the two sets: a 16-step segment of a
 // 512^2 grid holds ~3 GB per set.  nsets: 2 when there is more than one
 // segment (replay and adjoint overlap), else 1.
-int adj_alloc(harm_ctx* c, AdjWork& w, int nsteps, int nslots, int nsets)
+void adj_plan(harm_ctx* c, AdjWork& w, int nsteps, int nslots, int nsets)
 {
   const size_t pl = (size_t)c->gr.plane, P = NPR * pl * sizeof(double);
   for (int x = 0; x < nsets; x++) {
@@ -1044,6 +1053,7 @@ int adj_alloc(harm_ctx* c, AdjWork& w, int nsteps, int nslots, int nsets)
       }
     }
     double* plast = (double*)w.get(P);
+    w.pnext[x].clear();
     for (int m = 0; m < nslots; m++) w.pnext[x].push_back(m + 1 < nslots ? w.rec[x][m + 1].pn : plast);
   }
   w.sc_adj = (DevScalars*)w.get(sizeof(DevScalars));
@@ -1056,7 +1066,6 @@ int adj_alloc(harm_ctx* c, AdjWork& w, int nsteps, int nslots, int nsets)
   w.Le = (double*)w.get(pl * sizeof(double));
   w.dts = (double*)w.get((size_t)nsteps * sizeof(double));
   w.dot = (double*)w.get(dot_blocks(c) * sizeof(double));
-  return w.ok ? HARM_OK : HARM_ENOMEM;
 }
 
 void save_state(harm_ctx* c, const Saved& s)
@@ -1105,7 +1114,7 @@ void adjoint_substep(harm_ctx* c, AdjWork& w, const Rec& r, int sub, double* lam
 // step n's adjoint from its record r and its output state pout (p^{n+1}),
 // dt the step's (a.sc->dt): w.La = lambda_{n+1} -> lambda_n.  Fixed roles
 // (La in and out, Lb the midpoint state's adjoint, Lc the accumulator), so
-// that a slot's adjoint step can be captured once and replayed.
+// that a slot's adjoint step can be captured once and replayed (long runs).
 void adjoint_step(harm_ctx* c, AdjWork& w, const Rec& r, const double* pout, double wm, double we)
 {
   const StepArgs a = c->args();
@@ -1210,14 +1219,15 @@ int harm_run_fixed_dt(harm_ctx* c, const double* dts, int nsteps, double w_mass,
   if (!adjoint_supported(c)) return HARM_EINVAL;
   AdjWork w;
   const StepArgs a = c->args();
-  w.dts = (double*)w.get((size_t)nsteps * sizeof(double));
-  w.La = (double*)w.get((size_t)NPR * c->gr.plane * sizeof(double));
-  w.dot = (double*)w.get(dot_blocks(c) * sizeof(double));
-  if (!w.ok) return HARM_ENOMEM;
+  int rc = w.alloc([&] {
+    w.dts = (double*)w.get((size_t)nsteps * sizeof(double));
+    w.La = (double*)w.get((size_t)NPR * c->gr.plane * sizeof(double));
+    w.dot = (double*)w.get(dot_blocks(c) * sizeof(double));
+  });
+  if (rc) return rc;
   CK(cudaMemcpyAsync(w.dts, dts, (size_t)nsteps * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   bound_input(c);
-  int rc = zero_accumulators(c);
-  if (rc) return rc;
+  if ((rc = zero_accumulators(c)) != HARM_OK) return rc;
   if ((rc = harm_step(c, 0)) != HARM_OK) return rc;  // capture the step graph
   for (int n = 0; n < nsteps; n++) {
     k_set_dt<<<1, 1, 0, c->stream>>>(a, w.dts, n);
@@ -1236,14 +1246,20 @@ int harm_adjoint_run(harm_ctx* c, int nsteps, int checkpoint_every, double w_mas
   AdjWork w;
   const int nck = (nsteps + checkpoint_every - 1) / checkpoint_every;
   const int nsets = (nck > 1) ? 2 : 1;
-  int rc = adj_alloc(c, w, nsteps, std::min(checkpoint_every, nsteps), nsets);
-  if (rc) return rc;
   const size_t pl = (size_t)c->gr.plane, P = NPR * pl * sizeof(double);
   std::vector<Saved> ck(nck);
-  for (auto& x : ck) x = Saved{(double*)w.get(P), (double*)w.get(pl * sizeof(double))};
-  Saved fin{(double*)w.get(P), (double*)w.get(pl * sizeof(double))};
-  Saved in0{(double*)w.get(P), (double*)w.get(pl * sizeof(double))};
-  if (!w.ok) return HARM_ENOMEM;
+  Saved fin, in0;
+  int rc = w.alloc([&] {
+    adj_plan(c, w, nsteps, std::min(checkpoint_every, nsteps), nsets);
+    auto saved = [&] {
+      double* p = (double*)w.get(P);
+      return Saved{p, (double*)w.get(pl * sizeof(double))};
+    };
+    for (auto& x : ck) x = saved();
+    fin = saved();
+    in0 = saved();
+  });
+  if (rc) return rc;
   const StepArgs a = c->args();
   cudaStream_t s = c->stream;
   cudaEvent_t e0, e1, e2;
@@ -1275,7 +1291,7 @@ int harm_adjoint_run(harm_ctx* c, int nsteps, int checkpoint_every, double w_mas
   save_state(c, fin);
   // reverse, segment by segment: recompute the segment from its checkpoint,
   // recording every step, then the steps' adjoints in reverse order (both
-  // as per-slot graphs, captured on first use).  The replay of segment sg-1
+  // in long runs as per-slot graphs).  The replay of segment sg-1
   // (this context's stream, record set (sg-1) & 1) runs while the adjoint of
   // segment sg (stream sa, set sg & 1) does: they share only the geometry
   // (read) -- the adjoint's steps read their dt from their own scalars.  A
@@ -1323,17 +1339,28 @@ int harm_adjoint_run(harm_ctx* c, int nsteps, int checkpoint_every, double w_mas
     w.recg[x].assign(w.rec[x].size(), nullptr);
     w.adjg[x].assign(w.rec[x].size(), nullptr);
   }
+  // A slot's step is captured into a graph where the graph is launched often
+  // enough: capturing and instantiating one takes as long as issuing its ~30
+  // kernels a dozen times (256^2, 32 steps in two segments: 64 graphs were
+  // 0.1 s of a 0.28 s call whose kernels take 0.033 s); issued one by one
+  // they still stay ahead of the device (0.15 of 0.9 ms a step).
+  const bool graphs = (nck + nsets - 1) / nsets >= 16;
   auto replay = [&](int sg) -> int {
     const int x = sg & (nsets - 1), n0 = sg * checkpoint_every, len = std::min(checkpoint_every, nsteps - n0);
     load_state(c, ck[sg]);
     for (int m = 0; m < len; m++) {
-      if (!w.recg[x][m]) {
+      if (graphs && !w.recg[x][m]) {
         const Rec* r = &w.rec[x][m];
         const int rc2 = capture_graph(c, [r](harm_ctx* t) { return enqueue_step(t, nullptr, r); }, &w.recg[x][m]);
         if (rc2 != HARM_OK) return rc2;
       }
       k_set_dt<<<1, 1, 0, s>>>(a, w.dts, n0 + m);
-      CK(cudaGraphLaunch(w.recg[x][m], s));
+      if (graphs) {
+        CK(cudaGraphLaunch(w.recg[x][m], s));
+      } else {
+        const int rc2 = enqueue_step(c, nullptr, &w.rec[x][m]);
+        if (rc2 != HARM_OK) return rc2;
+      }
     }
     // the segment's last state, where its last step's adjoint reads it
     CK(cudaMemcpyAsync(w.pnext[x][len - 1], c->d_p, P, cudaMemcpyDeviceToDevice, s));
@@ -1350,7 +1377,7 @@ int harm_adjoint_run(harm_ctx* c, int nsteps, int checkpoint_every, double w_mas
       if ((rc = replay(sg - 1)) != HARM_OK) return rc;
     }
     for (int m = len - 1; m >= 0; m--) {
-      if (!w.adjg[x][m]) {
+      if (graphs && !w.adjg[x][m]) {
         const Rec* r = &w.rec[x][m];
         const double* po = w.pnext[x][m];
         AdjWork* wp = &w;
@@ -1361,8 +1388,10 @@ int harm_adjoint_run(harm_ctx* c, int nsteps, int checkpoint_every, double w_mas
         if (rc != HARM_OK) return rc;
       }
       k_set_dt<<<1, 1, 0, sa>>>(aa, w.dts, n0 + m);
-      CK(cudaGraphLaunch(w.adjg[x][m], sa));
+      if (graphs) CK(cudaGraphLaunch(w.adjg[x][m], sa));
+      else adjoint_step(&ca, w, w.rec[x][m], w.pnext[x][m], w_mass, w_em);
     }
+    CK(cudaGetLastError());
     CK(cudaEventRecord(ev_adj[x], sa));
   }
   // through the input's bound: ghost adjoints onto the active zones
