@@ -24,7 +24,6 @@
 #include <cudaTypedefs.h>
 
 namespace harm {
-__global__ void k_bsqflags(StepArgs a, const double* pv);
 __global__ void k_bound(StepArgs a, double* pv, int with_pflag);
 __global__ void k_poledeath(StepArgs a, double* pv);
 __global__ void k_gammacheck(StepArgs a, double* pv, int poledeath);
@@ -248,17 +247,12 @@ static int enqueue_step(harm_ctx* c, Timer* tm = nullptr, const Rec* rec = nullp
   // the active zones' in k_update (from the state it forms anyway) and the
   // one-zone ring's in k_emf (in the mixed form these FP64 flags are built
   // with contraction, like the rest of its kernels); the force-free step
-  // has none (k_bsqflags clears them).  (With the
-  // flux switch every flag of the DQZLOOP range is needed by the first
-  // substep's fluxes: each k_flux thread forms its zone's, which its faces
-  // use.)
+  // has none (they stay zero).  With the flux switch every flag of the
+  // DQZLOOP range is needed by the first substep's fluxes: each k_flux thread
+  // forms its zone's, which its faces use.
   const bool fuse_bsq = (c->cfg.eom == HARM_EOM_GRMHD) && !c->cfg.fluxadjust;
   // with the switch, the first substep's k_flux forms all of them
   const bool flags_in_flux = c->cfg.fluxadjust != 0;
-  if (!fuse_bsq && !flags_in_flux) {
-    k_bsqflags<<<grid2(n1 + 2, n2 + 2, b), b, 0, s>>>(a, c->d_p);
-    T.mark(s, KC_BSQ);
-  }
   bool step_ended = false;
   for (int sub = 0; sub < 2; sub++) {
     if (rec) {
@@ -303,6 +297,13 @@ static int enqueue_step(harm_ctx* c, Timer* tm = nullptr, const Rec* rec = nullp
       launch_bound_fix(mixed, grid2(n1 + 2 * NG, n2 + 2 * NG, b), b, s, a, pf, last ? 1 : 0);
       T.mark(s, KC_FIXA);
       if (last) step_ended = true;
+      continue;
+    }
+    if (ffde && sub == 1 && !poledeath && !c->cfg.currents) {
+      // the force-free star's last bound also ends the step
+      launch_bound_fix(mixed, grid2(n1 + 2 * NG, n2 + 2 * NG, b), b, s, a, pf, 1);
+      T.mark(s, KC_FIXA);
+      step_ended = true;
       continue;
     }
     k_bound<<<grid2(n1 + 2 * NG, n2 + 2 * NG, b), b, 0, s>>>(a, pf, 1);

@@ -18,49 +18,14 @@
 //                  the last substep its last block also ends the step
 //                  (horizon sums, new dt)
 // The adjoint's recording path, the force-free step and the currents use
-// k_bound, k_poledeath, k_gammacheck, k_fixup_apply, k_bsqflags, k_step_end.
+// k_bound, k_poledeath, k_gammacheck, k_fixup_apply, k_step_end.
 #include <cuda_runtime.h>
 #include "harm_step_impl.cuh"
 #include "harm_tryagain.cuh"
 
 namespace harm {
 
-// ---------------------------------------------------------------- flags
-// get_bsqflags, fixup.c:1197-1295 over the DQZLOOP range [-1,N1]x[-1,N2]
-// (with fluxadjust also the flux choice of each zone)
-__global__ void k_bsqflags(StepArgs a, const double* __restrict__ pv)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x - 1;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y - 1;
-  if (i > a.gr.n1 || j > a.gr.n2) return;
-  const long long z = a.gr.at(i, j);
-  if (a.pp.eom && !a.pp.fluxadjust) {  // the b^2 checks are GRMHD-only (fixup.c:1214-1233)
-    a.bsqf[z] = 0;
-    return;
-  }
-  double pr[NPR];
-#pragma unroll
-  for (int k = 0; k < NPR; k++) pr[k] = __ldg(pv + k * a.gr.plane + z);
-  Geo<double> g;
-  load_geo(a, CENT, z, g);
-  unsigned char b = 0;
-  if (!a.pp.eom) {
-    State<double> q;
-    state_of(pr, g, q);
-    b = bsq_flag(a, pr, q);
-  }
-  a.bsqf[z] = b;
-  if (a.pp.fluxadjust) {
-    // FLAGREALFLUX (fixup.c:1236-1245, 1284-1290): the Lorentz-factor flag
-    // joins the b^2 flags; where any is 2 the hydro fluxes step down from
-    // fluxmethod (HLL -> LAXF, not below LAXF)
-    const double gamma = gamma_of(pr, g);
-    const int f1 = (gamma > 2.0 * a.pp.gammadamp) ? 2 : ((gamma > a.pp.gammadamp) ? 1 : 0);
-    const int rf = ((b & 3) == 2 || f1 == 2 || (b >> 2) == 2) ? a.pp.fluxmethod - 1 : a.pp.fluxmethod;
-    a.fluxf[z] = (unsigned char)(rf < 0 ? 0 : rf);
-  }
-}
-
+// ---------------------------------------------------------------- inversions
 // utoprim_2d to its full iteration limit: without branches, or itself
 __device__ __forceinline__ int utoprim_2d_full(const double* U, const Geo<double>& g, double* pr, double gam,
                                                double gammafail, int* niter, double* nst, long long nss, bool resume)
@@ -377,14 +342,16 @@ __device__ __forceinline__ void bound_ghost(const StepArgs& a, double* pv, int i
   }
 }
 
-__global__ void k_bound(StepArgs a, double* pv, int with_pflag)
+__device__ __forceinline__ void bound_zone(const StepArgs& a, double* pv, int i, int j, int with_pflag)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x - NG;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y - NG;
   const int n1 = a.gr.n1, n2 = a.gr.n2;
   if (i >= n1 + NG || j >= n2 + NG) return;
   if (i >= 0 && i < n1 && j >= 0 && j < n2) return;
   bound_ghost<false>(a, pv, i, j, with_pflag);
+}
+__global__ void k_bound(StepArgs a, double* pv, int with_pflag)
+{
+  bound_zone(a, pv, blockIdx.x * blockDim.x + threadIdx.x - NG, blockIdx.y * blockDim.y + threadIdx.y - NG, with_pflag);
 }
 
 // The end of a GRMHD substep in one kernel: fixup_utoprim's repairs applied
@@ -407,6 +374,12 @@ __global__ void k_bound(StepArgs a, double* pv, int with_pflag)
 // POLEDEATH rows (x * 0 of a value already zeroed is the same zero) -- into
 // ubuf, and the last block to finish runs step_end_finish (the blocks count
 // themselves in sc->blocks_done).
+//
+// FFDE: the same end of the force-free star's step, whose last bound (ghost
+// zones and their pflags; there are no repairs) it runs: with it and without
+// clearing the b^2 flags that the form never sets, the step is 8 launches
+// instead of 10 (512 x 256 dipole 139.9 -> 135.3 us a step, mixed 108.0 ->
+// 103.1).
 __device__ __forceinline__ void bound_fix_zone(const StepArgs& a, double* pv, int i, int j)
 {
   const int n1 = a.gr.n1, n2 = a.gr.n2;
@@ -430,12 +403,14 @@ __device__ __forceinline__ void bound_fix_zone(const StepArgs& a, double* pv, in
   bound_ghost<true>(a, pv, i, j, 0);
 }
 
-template <typename FT>
+template <typename FT, bool FFDE>
 __global__ void k_bound_fix(StepArgs a, double* pv, int step_end, int hrows)
 {
   if ((int)blockIdx.y >= hrows) {
-    bound_fix_zone(a, pv, blockIdx.x * blockDim.x + threadIdx.x - NG,
-                   (blockIdx.y - hrows) * blockDim.y + threadIdx.y - NG);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x - NG;
+    const int j = (blockIdx.y - hrows) * blockDim.y + threadIdx.y - NG;
+    if (FFDE) bound_zone(a, pv, i, j, 1);
+    else bound_fix_zone(a, pv, i, j);
   } else {
     const int nt = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int j = (blockIdx.y * gridDim.x + blockIdx.x) * nt + tid;
@@ -443,7 +418,7 @@ __global__ void k_bound_fix(StepArgs a, double* pv, int step_end, int hrows)
       const long long pl = a.gr.plane, z = a.gr.at(0, j);
       double pr[NPR], t4[4];
 #pragma unroll
-      for (int k = 0; k < NPR; k++) pr[k] = srcv<true>(a, pv, z, k);
+      for (int k = 0; k < NPR; k++) pr[k] = srcv<!FFDE>(a, pv, z, k);
       if (a.pp.bc == 0 && (j == 0 || j == a.gr.n2 - 1)) {
         pr[U2] *= 0.;
         pr[B2] *= 0.;
@@ -472,8 +447,13 @@ void launch_bound_fix(int mixed, dim3 g, dim3 b, cudaStream_t s, const StepArgs&
 {
   const int hrows = step_end ? (a.gr.n2 + g.x * b.x * b.y - 1) / (g.x * b.x * b.y) : 0;
   g.y += hrows;
-  if (mixed) k_bound_fix<float><<<g, b, 0, s>>>(a, pv, step_end, hrows);
-  else k_bound_fix<double><<<g, b, 0, s>>>(a, pv, step_end, hrows);
+  if (a.pp.eom) {
+    if (mixed) k_bound_fix<float, true><<<g, b, 0, s>>>(a, pv, step_end, hrows);
+    else k_bound_fix<double, true><<<g, b, 0, s>>>(a, pv, step_end, hrows);
+  } else {
+    if (mixed) k_bound_fix<float, false><<<g, b, 0, s>>>(a, pv, step_end, hrows);
+    else k_bound_fix<double, false><<<g, b, 0, s>>>(a, pv, step_end, hrows);
+  }
 }
 
 // POLEDEATH on the first and last active x2 rows (bounds.fishmon.c:296-327)
