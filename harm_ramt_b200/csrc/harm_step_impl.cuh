@@ -311,25 +311,37 @@ __device__ __forceinline__ void side_x(EX& ex, const double* pr, const StateX& q
   x.vmin = (vp < vm) ? vp : vm;
 }
 
-// face_flux without branches: left and right point at the two interface
-// states (planes ks doubles apart), dir 1 or 2, base at the metric of the
-// face's location.  F and dtij are valid where ex.ok().
-template <bool FFDE, typename EX>
-__device__ __forceinline__ void face_flux_x(EX& ex, const StepArgs& a, const double* base, int dir, const double* left,
-                                            const double* right, int ks, double* F, double& dtij, int rf)
+// what a face reads of its location's metric: g_{mu nu}, g^{t mu}, g^{dir dir}
+// and sqrt(-g)
+struct FaceGeo {
+  double c[10], gcon[4], gdd, sg;
+};
+// loads that start where they are written (asm: the compiler would load each
+// value at its use, in small batches)
+__device__ __forceinline__ void load_face_geo(const StepArgs& a, int dir, long long z, FaceGeo& g)
 {
   const long long pl = a.gr.plane;
-  double c[10], gcon[4];
+  const double* b = a.geo + (long long)(dir == 1 ? FACE1 : FACE2) * GEO_PER_LOC * pl + z;
 #pragma unroll
-  for (int k = 0; k < 10; k++) c[k] = __ldg(base + k * pl);
+  for (int k = 0; k < 10; k++) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(g.c[k]) : "l"(b + k * pl));
 #pragma unroll
-  for (int k = 0; k < 4; k++) gcon[k] = __ldg(base + (10 + k) * pl);
-  const double gdd = __ldg(base + (dir == 1 ? 14 : 17) * pl), sg = __ldg(base + 20 * pl);
-  const double gd = (dir == 1) ? gcon[1] : gcon[2];
+  for (int k = 0; k < 4; k++) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(g.gcon[k]) : "l"(b + (10 + k) * pl));
+  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(g.gdd) : "l"(b + (dir == 1 ? 14 : 17) * pl));
+  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(g.sg) : "l"(b + 20 * pl));
+}
+
+// face_flux without branches: left and right point at the two interface
+// states (planes ks doubles apart), dir 1 or 2, g its metric.  F and dtij are
+// valid where ex.ok().
+template <bool FFDE, typename EX>
+__device__ __forceinline__ void face_flux_x(EX& ex, const StepArgs& a, const FaceGeo& g, int dir, const double* left,
+                                            const double* right, int ks, double* F, double& dtij, int rf)
+{
+  const double gd = (dir == 1) ? g.gcon[1] : g.gcon[2];
   const double gam = a.pp.gam, limit = (a.pp.gammamax <= 1.) ? 1.e300 : a.pp.gammamax;
   const int bd = (B1 - 1 + dir) * ks;
   const double Bd = 0.5 * (left[bd] + right[bd]);
-  const LapseX l = lapse_x(ex, gcon);
+  const LapseX l = lapse_x(ex, g.gcon);
   SideX sl, sr;
 #pragma unroll
   for (int s = 0; s < 2; s++) {
@@ -340,9 +352,9 @@ __device__ __forceinline__ void face_flux_x(EX& ex, const StepArgs& a, const dou
     if (dir == 1) p[B1] = Bd;
     else p[B2] = Bd;
     StateX q;
-    state_x(ex, p, c, l, limit, q);
+    state_x(ex, p, g.c, l, limit, q);
     sl = sr;
-    side_x<FFDE>(ex, p, q, dir, sg, gcon[0], gd, gdd, gam, sr);
+    side_x<FFDE>(ex, p, q, dir, g.sg, g.gcon[0], gd, g.gdd, gam, sr);
   }
   double cmin = rmin(sl.vmin, sr.vmin), cmax = rmax(sl.vmax, sr.vmax);
   cmin = fabs(rmax(0., -cmin));
@@ -474,8 +486,8 @@ __device__ __forceinline__ void flux_block_dt(const StepArgs& a, double dt1, dou
   dt2 = block_min(dt2, sh[1]);
   if (threadIdx.x == 0 && threadIdx.y == 0) {
     const int b = blockIdx.y * gridDim.x + blockIdx.x;
-    a.blockmin[b] = dt1;
-    a.blockmin[a.nblocks_flux + b] = dt2;
+    if (blockIdx.z == 0) a.blockmin[b] = dt1;
+    if (blockIdx.z == gridDim.z - 1) a.blockmin[a.nblocks_flux + b] = dt2;
   }
 }
 
@@ -631,7 +643,7 @@ __global__ void __launch_bounds__(32 * BY, (BY == FLUX_BY_SMALL) ? 5 : 1)
 // a row of a slot plane: 33 doubles, so that lanes in successive rows hit
 // successive banks
 constexpr int FLUX_SLOT_W = 33;
-template <bool PARA, bool FFDE, int BY>
+template <bool PARA, bool FFDE, int BY, bool SPLIT>
 __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
     k_flux_fp64(const __grid_constant__ StepArgs a, const __grid_constant__ CUtensorMap prim_map)
 {
@@ -649,6 +661,13 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
   const bool own = (tx > 0) || (blockIdx.x == 0);  // lane 0 of a later block repeats a zone
   const long long z = a.gr.at(in ? i : -1, in ? j : -1);
   double dt1 = 1.e9, dt2 = 1.e9;
+  // SPLIT: a layer of blocks for each direction (flux_launch_by)
+  const bool does1 = !SPLIT || blockIdx.z == 0, does2 = !SPLIT || blockIdx.z == 1;
+  // the first face's metric is on its way while the states are formed (8-row
+  // blocks: 1024^2 298 -> 291 us; the small grids of 4-row ones keep their
+  // metric in L2, and their steps were 2% slower with it)
+  FaceGeo g;
+  if (BY == FLUX_BY_LARGE) load_face_geo(a, does1 ? 1 : 2, z, g);
   __syncthreads();  // the barrier is initialised before anyone polls it
   if (!mbar_wait(&bar, 0)) {
     if (tx == 0 && ty == 0) report_fail(a.sc, a.phase0 + PH_FACE1, FAIL_TMA_TIMEOUT, zone_order(i, j));
@@ -662,13 +681,14 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
   for (int k = ty; k < NPR; k += BY) {
     const double* t = tz + (k * PS - ty * FLUX_TILE_W - tx);  // the block's first zone
     double* d = slot + (k * KS - ty * SW - tx);
-    {
+    if (does2) {
       double* d2 = d + 2 * NPR * KS + tx;
       row_states<PARA, BY + 1>(t + tx - FLUX_TILE_W, FLUX_TILE_W, [&](int c, double l, double r) {
         if (c > 0) d2[NPR * KS + (c - 1) * SW] = l;
         if (c < BY) d2[c * SW] = r;
       });
     }
+    if (!does1) continue;
     const int row = tx % BY, c0 = (tx / BY) * BY;
     d += row * SW + c0;
     row_states<PARA, BY>(t + row * FLUX_TILE_W + c0, 1, [&](int c, double l, double r) {
@@ -682,7 +702,7 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
     if (a.flags_here) {
       const int f = flux_flags_x(a, tz, PS, z);
       rf = f >> 8;
-      if (own) {
+      if (own && does1) {
         a.bsqf[z] = (unsigned char)(f & 255);
         a.fluxf[z] = (unsigned char)rf;
       }
@@ -698,6 +718,7 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
   for (int q = 0; q < 4; q++)
 #pragma unroll
     for (int k = U1; k <= B3; k++) {
+      if (!(q < 2 ? does1 : does2)) continue;
       // (volatile: these values are read again where they are used)
       const double v = *const_cast<const volatile double*>(slot + (q * NPR + k) * KS);
       const uint32_t t = hi_word(v) & 0x7fffffffu;
@@ -705,17 +726,17 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
     }
   const bool tiny = __any_sync(0xffffffffu, small);
   // both faces in one stretch of code; what it could not take comes after it
-  bool todo1 = in && i >= 0 && tx > 0, todo2 = in && j >= 0 && own;
+  bool todo1 = does1 && in && i >= 0 && tx > 0, todo2 = does2 && in && j >= 0 && own;
   auto faces = [&](auto ex0) {
 #pragma unroll
     for (int dir = 1; dir <= 2; dir++) {
       bool& todo = (dir == 1) ? todo1 : todo2;
       if (!todo) continue;
       const double* left = slot + (2 * dir - 2) * NPR * KS;
-      const double* base = a.geo + (long long)(dir == 1 ? FACE1 : FACE2) * GEO_PER_LOC * a.gr.plane + z;
       double Fx[NX], dtij;
+      if ((dir == 2 && does1) || BY != FLUX_BY_LARGE) load_face_geo(a, dir, z, g);
       auto ex = ex0;
-      face_flux_x<FFDE>(ex, a, base, dir, left, left + NPR * KS, KS, Fx, dtij, rf);
+      face_flux_x<FFDE>(ex, a, g, dir, left, left + NPR * KS, KS, Fx, dtij, rf);
       if (ex.ok()) {
         store_face_x(a, i, j, dir, z, Fx);
         if (dir == 1) dt1 = (dtij < dt1) ? dtij : dt1;
@@ -744,12 +765,19 @@ inline void flux_launch_by(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, co
   constexpr bool fp64 = sizeof(T) == 8;
   constexpr size_t sm = flux_tile_bytes(BY) + (fp64 ? 4 * NPR * BY * FLUX_SLOT_W * sizeof(double) : 0);
   void (*kern)(StepArgs, CUtensorMap);
-  if constexpr (fp64) kern = k_flux_fp64<PARA, FFDE, BY>;
+  // Where the blocks would take at most half of the SMs' slots (four 4-row
+  // blocks each), each direction gets a layer of blocks of its own, and a
+  // block half the work: a step of the 64^2 torus 71.3 -> 65.3 us, 128^2 79.6
+  // -> 75.2, 245 x 131 90.9 -> 86.2 (the next size up fills the SMs anyway).
+  constexpr bool small = fp64 && BY == FLUX_BY_SMALL;
+  if (small && g.x * g.y <= 2 * 148) g.z = 2;
+  if constexpr (small) kern = (g.z == 2) ? k_flux_fp64<PARA, FFDE, BY, true> : k_flux_fp64<PARA, FFDE, BY, false>;
+  else if constexpr (fp64) kern = k_flux_fp64<PARA, FFDE, BY, false>;
   else kern = k_flux<T, PARA, FFDE, BY>;
-  static bool attr = false;
-  if (!attr) {
+  static bool attr[2] = {false, false};
+  if (!attr[g.z - 1]) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    attr = true;
+    attr[g.z - 1] = true;
   }
   kern<<<g, b, sm, s>>>(a, map);
 }
