@@ -72,6 +72,7 @@ struct DevScalars {
   double clastdt;        // currents: dt of the previous call (its static lastdt)
   int chk_multi;         // substeps whose check-solution sweep needed rounds after the first
   unsigned blocks_done;  // blocks of k_bound_fix finished (its last block ends the step; reset by that block)
+  unsigned terms_done;   // its blocks of horizon terms finished (the last one sums them; reset by it)
 };
 
 struct StepArgs {

@@ -368,18 +368,22 @@ __global__ void k_bound(StepArgs a, double* pv, int with_pflag)
 //
 // With step_end set (after the last substep) the grid starts with `hrows`
 // extra rows of blocks (launched first, so that their latency overlaps the
-// zones' work): their threads form the horizon terms of rows j from the
-// final state of zone (0, j) -- the value its own thread writes in this
-// kernel: the repair buffer's or pv's, times 0 for u~2 and B2 on the
-// POLEDEATH rows (x * 0 of a value already zeroed is the same zero) -- into
-// ubuf, and the last block to finish runs step_end_finish (the blocks count
-// themselves in sc->blocks_done).
+// zones' work): the threads of the first of them form the horizon terms of
+// rows j from the final state of zone (0, j) -- the value its own thread
+// writes in this kernel: the repair buffer's or pv's, times 0 for u~2 and B2
+// on the POLEDEATH rows (x * 0 of a value already zeroed is the same zero) --
+// into ubuf, and the last of them to finish sums them; one more block forms
+// the new dt.  The last block of the grid to finish commits the step's scalars
+// (blocks count themselves in sc->terms_done and sc->blocks_done).  Summing
+// and the Courant minima in the last block of the grid instead, after all
+// others, put their whole latency at the end of the step (512^2 346.8 -> 343.3
+// us a step, 1024^2 1067 -> 1050, the dipole 132.9 -> 131.3).
 //
 // FFDE: the same end of the force-free star's step, whose last bound (ghost
 // zones and their pflags; there are no repairs) it runs: with it and without
 // clearing the b^2 flags that the form never sets, the step is 8 launches
-// instead of 10 (512 x 256 dipole 139.9 -> 135.3 us a step, mixed 108.0 ->
-// 103.1).
+// instead of 10 (512 x 256 dipole 139.2 -> 133.5 us a step, mixed 107.6 ->
+// 102.8).
 __device__ __forceinline__ void bound_fix_zone(const StepArgs& a, double* pv, int i, int j)
 {
   const int n1 = a.gr.n1, n2 = a.gr.n2;
@@ -403,6 +407,23 @@ __device__ __forceinline__ void bound_fix_zone(const StepArgs& a, double* pv, in
   bound_ghost<true>(a, pv, i, j, 0);
 }
 
+// every thread of a block: whether the block is the last of n to come here
+// (what the others wrote before is then visible)
+__device__ __forceinline__ bool last_to_finish(unsigned* count, unsigned n)
+{
+  __shared__ int last;
+  __syncthreads();
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
+    __threadfence();
+    last = (atomicAdd(count, 1u) == n - 1);
+  }
+  __syncthreads();
+  const bool mine = last != 0;
+  if (mine) __threadfence();
+  __syncthreads();  // `last` may be used again
+  return mine;
+}
+
 template <typename FT, bool FFDE>
 __global__ void k_bound_fix(StepArgs a, double* pv, int step_end, int hrows)
 {
@@ -413,7 +434,7 @@ __global__ void k_bound_fix(StepArgs a, double* pv, int step_end, int hrows)
     else bound_fix_zone(a, pv, i, j);
   } else {
     const int nt = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const int j = (blockIdx.y * gridDim.x + blockIdx.x) * nt + tid;
+    const int tb = blockIdx.y * gridDim.x + blockIdx.x, nterm = (a.gr.n2 + nt - 1) / nt, j = tb * nt + tid;
     if (j < a.gr.n2) {
       const long long pl = a.gr.plane, z = a.gr.at(0, j);
       double pr[NPR], t4[4];
@@ -427,25 +448,26 @@ __global__ void k_bound_fix(StepArgs a, double* pv, int step_end, int hrows)
 #pragma unroll
       for (int k = 0; k < 4; k++) a.ubuf[k * pl + j] = t4[k];
     }
+    if (tb < nterm) {
+      if (last_to_finish(&a.sc->terms_done, nterm)) {
+        step_sums<true>(a, a.ubuf, a.gr.plane);
+        if (tid == 0) a.sc->terms_done = 0;
+      }
+    } else if (tb == nterm) {
+      step_dt(a);
+    }
   }
   if (!step_end) return;
-  __shared__ int last;
-  __syncthreads();
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    __threadfence();
-    const unsigned nb = gridDim.x * gridDim.y;
-    last = (atomicAdd(&a.sc->blocks_done, 1u) == nb - 1);
+  if (last_to_finish(&a.sc->blocks_done, gridDim.x * gridDim.y) && threadIdx.x == 0 && threadIdx.y == 0) {
+    step_commit(a);
+    a.sc->blocks_done = 0;
   }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  step_end_finish<true>(a, a.ubuf, a.gr.plane);
-  if (threadIdx.x == 0 && threadIdx.y == 0) a.sc->blocks_done = 0;
 }
 
 void launch_bound_fix(int mixed, dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, double* pv, int step_end)
 {
-  const int hrows = step_end ? (a.gr.n2 + g.x * b.x * b.y - 1) / (g.x * b.x * b.y) : 0;
+  // blocks of horizon terms and the one that forms dt, in rows of g.x
+  const int nt = b.x * b.y, hrows = step_end ? ((a.gr.n2 + nt - 1) / nt + 1 + g.x - 1) / g.x : 0;
   g.y += hrows;
   if (a.pp.eom) {
     if (mixed) k_bound_fix<float, true><<<g, b, 0, s>>>(a, pv, step_end, hrows);

@@ -1393,17 +1393,18 @@ __device__ __forceinline__ void horizon_terms(const StepArgs& a, const double* p
   t4[3] = -(q.bcon[1]) * (q.bcov[0]) * surgdet;
 }
 
-// The end of a step, by every thread of one block, after the horizon terms
-// of every row j sit in t[k * ts + j] (k < 4): their sums in j order as the
-// reference's loop adds them (so the sums are exact), pcum += pdot * dt
-// (diag.c:576-833); then the new dt from the flux blocks' Courant minima
-// (advance.c:190, step_ch.c:174-183) and t += dt.  L2: the terms were
-// written by other blocks of the same kernel (read past L1).
+// The end of a step in three parts.  step_sums, by every thread of one
+// block, after the horizon terms of every row j sit in t[k * ts + j] (k < 4):
+// their sums in j order as the reference's loop adds them (so the sums are
+// exact), pcum += pdot * dt (diag.c:576-833).  step_dt, by one block: the new
+// dt from the flux blocks' Courant minima (advance.c:190, step_ch.c:174-183).
+// step_commit, one thread, after both and after everything that reads the
+// step's scalars: t += dt and the new dt.  L2: the terms were written by other
+// blocks of the same kernel (read past L1).
 template <bool L2>
-__device__ __forceinline__ void step_end_finish(const StepArgs& a, const double* t, long long ts)
+__device__ __forceinline__ void step_sums(const StepArgs& a, const double* t, long long ts)
 {
   constexpr int CHUNK = 256;
-  __shared__ double sh[2][32];
   __shared__ double acc[4];
   __shared__ double stage[4][CHUNK + 1];  // rows one double apart in banks: the four adding lanes do not conflict
   const int tid = threadIdx.y * blockDim.x + threadIdx.x, nt = blockDim.x * blockDim.y;
@@ -1444,6 +1445,12 @@ __device__ __forceinline__ void step_end_finish(const StepArgs& a, const double*
     sc->hz[5] += acc[1] * sc->dt;
     sc->hz[6] += (acc[2] + acc[3]) * sc->dt;
   }
+}
+
+__device__ __forceinline__ void step_dt(const StepArgs& a)
+{
+  __shared__ double sh[2][32];
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x, nt = blockDim.x * blockDim.y;
   double m1 = 1.e9, m2 = 1.e9;
 #pragma unroll 4
   for (int b = tid; b < a.nblocks_flux; b += nt) {
@@ -1453,22 +1460,24 @@ __device__ __forceinline__ void step_end_finish(const StepArgs& a, const double*
   }
   m1 = block_min(m1, sh[0]);
   m2 = block_min(m2, sh[1]);
-  if (tid == 0) {
-    DevScalars* s = a.sc;
-    double ndt = a.pp.defcon * 1. / (1. / m1 + 1. / m2);
-    s->ndt = ndt;
-    const bool moved = s->dt > 0.;
-    s->t += s->dt;
-    s->realnstep += 1;
-    if (ndt > a.pp.safe * s->dt) ndt = a.pp.safe * s->dt;
-    s->dt = ndt;
-    if (moved) s->dt_free = ndt;  // a step at dt = 0 (past the end time) keeps the last one
-    if (s->t + s->dt > a.pp.tf) s->dt = a.pp.tf - s->t;
-  }
+  if (tid == 0) a.sc->ndt = a.pp.defcon * 1. / (1. / m1 + 1. / m2);
+}
+
+__device__ __forceinline__ void step_commit(const StepArgs& a)
+{
+  DevScalars* s = a.sc;
+  double ndt = __ldcg(&s->ndt);
+  const bool moved = s->dt > 0.;
+  s->t += s->dt;
+  s->realnstep += 1;
+  if (ndt > a.pp.safe * s->dt) ndt = a.pp.safe * s->dt;
+  s->dt = ndt;
+  if (moved) s->dt_free = ndt;  // a step at dt = 0 (past the end time) keeps the last one
+  if (s->t + s->dt > a.pp.tf) s->dt = a.pp.tf - s->t;
 }
 
 // After the last substep, one block: the horizon terms of every row j (into
-// the inversion scratch ubuf, idle by now), then step_end_finish.
+// the inversion scratch ubuf, idle by now), then the three parts.
 constexpr int STEP_END_THREADS = 512;
 template <typename FT>
 __global__ void __launch_bounds__(STEP_END_THREADS) k_step_end(StepArgs a, const double* __restrict__ pv)
@@ -1484,7 +1493,10 @@ __global__ void __launch_bounds__(STEP_END_THREADS) k_step_end(StepArgs a, const
     for (int k = 0; k < 4; k++) a.ubuf[k * pl + j] = t4[k];
   }
   __syncthreads();
-  step_end_finish<false>(a, a.ubuf, pl);
+  step_sums<false>(a, a.ubuf, pl);
+  step_dt(a);
+  __syncthreads();
+  if (threadIdx.x == 0) step_commit(a);
 }
 
 }  // namespace harm
