@@ -81,6 +81,7 @@ struct harm_ctx {
   int nblocks_flux;
   int flux_by;       // k_flux rows per block (flux_rows)
   bool geo_ok;
+  int sparse;        // the uploaded metric is of the sparse form (SP in harm_step_impl.cuh)
   cudaGraph_t graph;
   cudaGraphExec_t gexec;
   bool have_graph;
@@ -110,6 +111,8 @@ struct harm_ctx {
     a.pp.tf = cfg.tf;
     a.geo = d_geo;
     a.geo32 = d_geo32;
+    a.sparse = sparse;
+    a.geo_full = reinterpret_cast<const int*>(d_geo + GEO_NPLANES * gr.plane);
     a.F1 = d_F1;
     a.F2 = d_F2;
     a.emf = d_emf;
@@ -354,6 +357,15 @@ static int enqueue_step(harm_ctx* c, Timer* tm = nullptr, const Rec* rec = nullp
   return cudaGetLastError() == cudaSuccess ? HARM_OK : HARM_ECUDA;
 }
 
+static void drop_graph(harm_ctx* c)
+{
+  if (c->have_graph) {
+    cudaGraphExecDestroy(c->gexec);
+    cudaGraphDestroy(c->graph);
+    c->have_graph = false;
+  }
+}
+
 extern "C" {
 
 const char* harm_error_string(int code)
@@ -409,7 +421,7 @@ int harm_create(const harm_config* cfg, void* stream, harm_ctx** out)
   bool ok = true;
   ok &= cudaMalloc(&c->d_p, NPR * pd) == cudaSuccess;
   ok &= cudaMalloc(&c->d_pk0, NPR * pd) == cudaSuccess;
-  ok &= cudaMalloc(&c->d_geo, GEO_NPLANES * pd) == cudaSuccess;
+  ok &= cudaMalloc(&c->d_geo, GEO_NPLANES * pd + 256) == cudaSuccess;  // (+ geo_full)
   if (cfg->precision == HARM_PREC_MIXED)
     ok &= cudaMalloc(&c->d_geo32, 2 * GEO_PER_LOC * (size_t)c->gr.plane * sizeof(float)) == cudaSuccess;
   ok &= cudaMalloc(&c->d_F1, NPR * pd) == cudaSuccess;
@@ -440,7 +452,7 @@ int harm_create(const harm_config* cfg, void* stream, harm_ctx** out)
   }
   cudaMemsetAsync(c->d_p, 0, NPR * pd, c->stream);
   cudaMemsetAsync(c->d_pk0, 0, NPR * pd, c->stream);
-  cudaMemsetAsync(c->d_geo, 0, GEO_NPLANES * pd, c->stream);
+  cudaMemsetAsync(c->d_geo, 0, GEO_NPLANES * pd + 256, c->stream);
   cudaMemsetAsync(c->d_F1, 0, NPR * pd, c->stream);
   cudaMemsetAsync(c->d_F2, 0, NPR * pd, c->stream);
   cudaMemsetAsync(c->d_emf, 0, pd, c->stream);
@@ -497,6 +509,9 @@ int harm_upload_geometry(harm_ctx* c, const double* gcov, const double* gcon, co
   const int n1m = c->n1m, n2m = c->n2m;
   const long long pl = c->gr.plane;
   std::vector<double> h((size_t)GEO_NPLANES * pl, 0.0);
+  // the sparse form: g_{t2}, g_{12}, g_{23} and g^{t2}, g^{t3}, g^{12}, g^{23}
+  // exactly zero at every x1 and x2 face and centre
+  int full = 0;
   for (int ii = 0; ii < n1m; ii++)
     for (int jj = 0; jj < n2m; jj++) {
       const long long zr = (long long)ii * n2m + jj;                 // reference zone
@@ -513,6 +528,9 @@ int harm_upload_geometry(harm_ctx* c, const double* gcov, const double* gcon, co
             h[((size_t)loc * GEO_PER_LOC + 10 + sym(a, b)) * pl + zd] = gn[a * 4 + b];
           }
         h[((size_t)loc * GEO_PER_LOC + 20) * pl + zd] = gdet[zr * 4 + loc];
+        if (loc != CORN)
+          full |= !(gv[2] == 0. && gv[6] == 0. && gv[11] == 0. && gn[2] == 0. && gn[3] == 0. && gn[6] == 0. &&
+                    gn[11] == 0.);
       }
       const double* cn = conn + zr * 64;
       for (int k = 0; k < 4; k++)
@@ -525,6 +543,9 @@ int harm_upload_geometry(harm_ctx* c, const double* gcov, const double* gcon, co
       h[(size_t)(GEO_FLOOR + 1) * pl + zd] = floors[zr * 2 + 1];
     }
   CK(cudaMemcpyAsync(c->d_geo, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  // the kernels chosen for a captured step see a metric of the other form by
+  // this flag (an ensemble's graph); the context's own graph is made again
+  CK(cudaMemcpyAsync(c->d_geo + GEO_NPLANES * pl, &full, sizeof(full), cudaMemcpyHostToDevice, c->stream));
   std::vector<float> h32;
   if (c->d_geo32) {
     // FP32 copies of the two face locations (FACE1, FACE2 are the first 42 planes)
@@ -533,6 +554,8 @@ int harm_upload_geometry(harm_ctx* c, const double* gcov, const double* gcon, co
     CK(cudaMemcpyAsync(c->d_geo32, h32.data(), h32.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
   }
   CK(cudaStreamSynchronize(c->stream));
+  if (c->sparse != !full) drop_graph(c);
+  c->sparse = !full;
   c->geo_ok = true;
   return HARM_OK;
 }
@@ -825,15 +848,6 @@ int harm_write_dump(harm_ctx* c, const char* path, const harm_dump_header* hdr, 
   for (auto& s : chunk) ok &= fwrite(s.data(), 1, s.size(), f) == s.size();
   ok &= fclose(f) == 0;
   return ok ? HARM_OK : HARM_EINVAL;
-}
-
-static void drop_graph(harm_ctx* c)
-{
-  if (c->have_graph) {
-    cudaGraphExecDestroy(c->gexec);
-    cudaGraphDestroy(c->graph);
-    c->have_graph = false;
-  }
 }
 
 int harm_set_tiles(harm_ctx* c, const harm_tiles* t)

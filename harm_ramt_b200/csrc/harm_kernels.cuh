@@ -79,6 +79,8 @@ struct StepArgs {
   Grid gr;
   Params pp;
   const double* geo;     // GEO_NPLANES planes
+  const int* geo_full;   // nonzero: the uploaded metric is not of the sparse form
+  int sparse;            // kernels for the sparse form (SP in harm_step_impl.cuh) are chosen
   const float* geo32;    // mixed precision: FACE1 and FACE2 geometry (2 x 21 float planes)
   double* F1;            // 8 planes (of float in mixed precision)
   double* F2;            // 8 planes (of float in mixed precision)

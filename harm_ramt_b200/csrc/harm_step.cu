@@ -34,7 +34,7 @@ __device__ __forceinline__ int utoprim_2d_full(const double* U, const Geo<double
 #pragma unroll
   for (int k = 0; k < NPR; k++) p[k] = pr[k];
   ExactTiny ex;
-  const int pfl = utoprim_2d_x(ex, U, g.gcov, g.gcon, g.g, p, gam, gammafail, niter, 200, nst, nss, resume);
+  const int pfl = utoprim_2d_x<false>(ex, U, g.gcov, g.gcon, g.g, p, gam, gammafail, niter, 200, nst, nss, resume);
   if (!ex.ok()) return utoprim_2d(U, g, pr, gam, gammafail, niter, 200, nst, nss, resume);
 #pragma unroll
   for (int k = 0; k < NPR; k++) pr[k] = p[k];
@@ -1017,15 +1017,22 @@ __global__ void k_planes_to_ref(StepArgs a, const double* __restrict__ pv, doubl
 // launchers of the templated kernels: the FP64 instantiations here, the
 // mixed-precision ones in harm_step_mixed.cu
 
+template <bool SP>
+static void flux_fp64(int para, int ffde, dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& prim_map)
+{
+  if (ffde) {
+    if (para) flux_rows_launch<double, true, true, SP>(g, b, s, a, prim_map);
+    else flux_rows_launch<double, false, true, SP>(g, b, s, a, prim_map);
+  } else if (para) flux_rows_launch<double, true, false, SP>(g, b, s, a, prim_map);
+  else flux_rows_launch<double, false, false, SP>(g, b, s, a, prim_map);
+}
+
 void launch_flux(int para, int mixed, int ffde, dim3 g, dim3 b, cudaStream_t s, const StepArgs& a,
                  const CUtensorMap& prim_map)
 {
   if (mixed) launch_flux_mixed(para, ffde, g, b, s, a, prim_map);
-  else if (ffde) {
-    if (para) flux_rows_launch<double, true, true>(g, b, s, a, prim_map);
-    else flux_rows_launch<double, false, true>(g, b, s, a, prim_map);
-  } else if (para) flux_rows_launch<double, true, false>(g, b, s, a, prim_map);
-  else flux_rows_launch<double, false, false>(g, b, s, a, prim_map);
+  else if (a.sparse) flux_fp64<true>(para, ffde, g, b, s, a, prim_map);
+  else flux_fp64<false>(para, ffde, g, b, s, a, prim_map);
 }
 
 void launch_emf(int mixed, dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const double* pv)

@@ -165,18 +165,74 @@ __device__ __forceinline__ void face_flux(const StepArgs& a, int i, int j, int d
 // Where the templates branch (a Lorentz limit, a wavespeed outside its
 // bounds) ex.ok() is false and the face goes through face_flux.
 
+// SP: a metric that couples x2 to nothing else and t not to phi in g^{mu nu}
+// (g_{t2} = g_{12} = g_{23} = 0, g^{t2} = g^{t3} = g^{12} = g^{23} = 0 at every
+// face and centre: Kerr-Schild on a grid stretched along x1 and x2, flat
+// space), found when the geometry is uploaded.  Its sums leave out the terms
+// that are a finite value times an exact zero, and those planes are not read:
+// k_flux of the 512^2 torus 87 -> 79.5 us, 1024^2 292 -> 268, the 512 x 256
+// dipole 40 -> 34.5; k_update 51 and 58 -> 49 and 53, 1024^2 178 -> 160.
+constexpr int SP_COV = (1 << 2) | (1 << 5) | (1 << 8), SP_CON = SP_COV | (1 << 3);
+template <bool SP>
+__device__ __forceinline__ void lower_cov(const double* v, const double* c, double* w)
+{
+  if (!SP) {
+    lower_v(v, c, w);
+    return;
+  }
+  w[0] = c[0] * v[0] + c[1] * v[1] + c[3] * v[3];
+  w[1] = c[1] * v[0] + c[4] * v[1] + c[6] * v[3];
+  w[2] = c[7] * v[2];
+  w[3] = c[3] * v[0] + c[6] * v[1] + c[9] * v[3];
+}
+template <bool SP>
+__device__ __forceinline__ void raise_con(const double* v, const double* g, double* w)
+{
+  if (!SP) {
+    lower_v(v, g, w);
+    return;
+  }
+  w[0] = g[0] * v[0] + g[1] * v[1];
+  w[1] = g[1] * v[0] + g[4] * v[1] + g[6] * v[3];
+  w[2] = g[7] * v[2];
+  w[3] = g[6] * v[1] + g[9] * v[3];
+}
+// the space part of lower_cov for a vector without a time component
+template <bool SP>
+__device__ __forceinline__ void lower_space(const double* b, const double* c, double* w)
+{
+  if (SP) {
+    w[0] = c[4] * b[0] + c[6] * b[2];
+    w[1] = c[7] * b[1];
+    w[2] = c[6] * b[0] + c[9] * b[2];
+  } else {
+    w[0] = c[4] * b[0] + c[5] * b[1] + c[6] * b[2];
+    w[1] = c[5] * b[0] + c[7] * b[1] + c[8] * b[2];
+    w[2] = c[6] * b[0] + c[8] * b[1] + c[9] * b[2];
+  }
+}
+// the q^2 of gamma_calc
+template <bool SP>
+__device__ __forceinline__ double qsq_x(const double* pr, const double* c)
+{
+  const double d = c[4] * pr[U1] * pr[U1] + c[7] * pr[U2] * pr[U2] + c[9] * pr[U3] * pr[U3];
+  if (SP) return d + 2. * (c[6] * pr[U1] * pr[U3]);
+  return d + 2. * (c[5] * pr[U1] * pr[U2] + c[6] * pr[U1] * pr[U3] + c[8] * pr[U2] * pr[U3]);
+}
+
 // lapse and shift of a location, as ucon_calc_rel4vel forms them
 struct LapseX {
   Recip alpha;
   double beta[3];
 };
+template <bool SP>
 __device__ __forceinline__ LapseX lapse_x(Exact& ex, const double* gcon)
 {
   LapseX l;
   const double alpha = Exact::quot(1., ex.rcp(ex.sqrt_of(-gcon[0])));
   l.alpha = ex.rcp(alpha);
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
+  for (int k = 0; k < (SP ? 1 : 3); k++) {
     l.beta[k] = gcon[1 + k] * alpha * alpha;
     ex.numerator<-600>(l.beta[k]);
   }
@@ -188,24 +244,23 @@ struct StateX : State<double> {
   double bsq, gamma;
 };
 // get_state; limit: GAMMAMAX where the caller limits the Lorentz factor first
-template <typename EX>
+template <bool SP, typename EX>
 __device__ __forceinline__ void state_x(EX& ex, const double* pr, const double* c, const LapseX& l, double limit,
                                         StateX& q)
 {
-  const double qsq = c[4] * pr[U1] * pr[U1] + c[7] * pr[U2] * pr[U2] + c[9] * pr[U3] * pr[U3] +
-                     2. * (c[5] * pr[U1] * pr[U2] + c[6] * pr[U1] * pr[U3] + c[8] * pr[U2] * pr[U3]);
-  const double gamma = ex.sqrt_of(1. + qsq);
+  const double gamma = ex.sqrt_of(1. + qsq_x<SP>(pr, c));
   ex.need(gamma <= limit);
   q.gamma = gamma;
   q.ucon[0] = Exact::quot(gamma, l.alpha);
 #pragma unroll
-  for (int k = 0; k < 3; k++) q.ucon[1 + k] = pr[U1 + k] - Exact::quot(gamma * l.beta[k], l.alpha);
-  lower_v(q.ucon, c, q.ucov);
+  for (int k = 0; k < 3; k++)
+    q.ucon[1 + k] = (SP && k > 0) ? pr[U1 + k] : pr[U1 + k] - Exact::quot(gamma * l.beta[k], l.alpha);
+  lower_cov<SP>(q.ucon, c, q.ucov);
   q.bcon[0] = pr[B1] * q.ucov[1] + pr[B2] * q.ucov[2] + pr[B3] * q.ucov[3];
   q.ut = ex.rcp(q.ucon[0]);
 #pragma unroll
   for (int k = 1; k < 4; k++) q.bcon[k] = ex.div(pr[B1 - 1 + k] + q.bcon[0] * q.ucon[k], q.ut);
-  lower_v(q.bcon, c, q.bcov);
+  lower_cov<SP>(q.bcon, c, q.bcov);
   q.bsq = dot4(q.bcon, q.bcov);
 }
 
@@ -250,7 +305,7 @@ struct SideX {
 
 // primtoflux in direction dir (1 or 2) and in time, and vchar; sg: sqrt(-g);
 // gd, gdd: g^{t dir} and g^{dir dir}
-template <bool FFDE, typename EX>
+template <bool FFDE, bool SP, typename EX>
 __device__ __forceinline__ void side_x(EX& ex, const double* pr, const StateX& q, int dir, double sg, double gtt,
                                        double gd, double gdd, double gam, SideX& x)
 {
@@ -301,7 +356,7 @@ __device__ __forceinline__ void side_x(EX& ex, const double* pr, const StateX& q
   const double Au = d1 ? q.ucon[1] : q.ucon[2], Bu = q.ucon[0];
   const double Au2 = Au * Au, Bu2 = Bu * Bu, AuBu = Au * Bu;
   const double A = Bu2 - (gtt + Bu2) * cms2;
-  const double B = 2. * (AuBu - (gd + AuBu) * cms2);
+  const double B = 2. * (AuBu - ((SP && !d1) ? AuBu : gd + AuBu) * cms2);
   const double C = Au2 - (gdd + Au2) * cms2;
   const double s = ex.sqrt_of(B * B - 4. * A * C);
   const Recip A2 = ex.rcp(2. * A);
@@ -318,14 +373,16 @@ struct FaceGeo {
 };
 // loads that start where they are written (asm: the compiler would load each
 // value at its use, in small batches)
+template <bool SP>
 __device__ __forceinline__ void load_face_geo(const StepArgs& a, int dir, long long z, FaceGeo& g)
 {
   const long long pl = a.gr.plane;
   const double* b = a.geo + (long long)(dir == 1 ? FACE1 : FACE2) * GEO_PER_LOC * pl + z;
 #pragma unroll
-  for (int k = 0; k < 10; k++) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(g.c[k]) : "l"(b + k * pl));
+  for (int k = 0; k < 10; k++)
+    if (!SP || !(SP_COV >> k & 1)) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(g.c[k]) : "l"(b + k * pl));
 #pragma unroll
-  for (int k = 0; k < 4; k++) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(g.gcon[k]) : "l"(b + (10 + k) * pl));
+  for (int k = 0; k < (SP ? 2 : 4); k++) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(g.gcon[k]) : "l"(b + (10 + k) * pl));
   asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(g.gdd) : "l"(b + (dir == 1 ? 14 : 17) * pl));
   asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(g.sg) : "l"(b + 20 * pl));
 }
@@ -333,15 +390,15 @@ __device__ __forceinline__ void load_face_geo(const StepArgs& a, int dir, long l
 // face_flux without branches: left and right point at the two interface
 // states (planes ks doubles apart), dir 1 or 2, g its metric.  F and dtij are
 // valid where ex.ok().
-template <bool FFDE, typename EX>
+template <bool FFDE, bool SP, typename EX>
 __device__ __forceinline__ void face_flux_x(EX& ex, const StepArgs& a, const FaceGeo& g, int dir, const double* left,
                                             const double* right, int ks, double* F, double& dtij, int rf)
 {
-  const double gd = (dir == 1) ? g.gcon[1] : g.gcon[2];
+  const double gd = (dir == 1) ? g.gcon[1] : (SP ? 0. : g.gcon[2]);
   const double gam = a.pp.gam, limit = (a.pp.gammamax <= 1.) ? 1.e300 : a.pp.gammamax;
   const int bd = (B1 - 1 + dir) * ks;
   const double Bd = 0.5 * (left[bd] + right[bd]);
-  const LapseX l = lapse_x(ex, g.gcon);
+  const LapseX l = lapse_x<SP>(ex, g.gcon);
   SideX sl, sr;
 #pragma unroll
   for (int s = 0; s < 2; s++) {
@@ -352,9 +409,9 @@ __device__ __forceinline__ void face_flux_x(EX& ex, const StepArgs& a, const Fac
     if (dir == 1) p[B1] = Bd;
     else p[B2] = Bd;
     StateX q;
-    state_x(ex, p, g.c, l, limit, q);
+    state_x<SP>(ex, p, g.c, l, limit, q);
     sl = sr;
-    side_x<FFDE>(ex, p, q, dir, g.sg, g.gcon[0], gd, g.gdd, gam, sr);
+    side_x<FFDE, SP>(ex, p, q, dir, g.sg, g.gcon[0], gd, g.gdd, gam, sr);
   }
   double cmin = rmin(sl.vmin, sr.vmin), cmax = rmax(sl.vmax, sr.vmax);
   cmin = fabs(rmax(0., -cmin));
@@ -527,7 +584,7 @@ static __device__ __noinline__ int flux_flags_x(const StepArgs& a, const double*
   for (int k = 0; k < 4; k++) gcon[k] = __ldg(base + (10 + k) * a.gr.plane);
   Exact ex;
   StateX q;
-  state_x(ex, pr, c, lapse_x(ex, gcon), 1.e300, q);
+  state_x<false>(ex, pr, c, lapse_x<false>(ex, gcon), 1.e300, q);
   const unsigned char b = bsq_flag_x(ex, a, pr, q.bsq);
   if (a.pp.eom || !ex.ok()) return flux_flags(a, tz, ps, z);
   const int f1 = (q.gamma > 2.0 * a.pp.gammadamp) ? 2 : ((q.gamma > a.pp.gammadamp) ? 1 : 0);
@@ -623,7 +680,7 @@ __global__ void __launch_bounds__(32 * BY, (BY == FLUX_BY_SMALL) ? 5 : 1)
 }
 
 // FP64 faces.  FP64 issue and latency bound: 2080 FP64-pipe instructions a
-// zone at 128 registers (16 warps per SM).  What the layout is for:
+// zone (1900 with the sparse metric) at 128 registers (16 warps per SM).  What the layout is for:
 //  * all interface states are formed first, into shared memory (four slots a
 //    zone: the left and right state of its x1 and x2 face).  A warp takes one
 //    variable of the whole block and walks along the zones, so each slope and
@@ -643,7 +700,7 @@ __global__ void __launch_bounds__(32 * BY, (BY == FLUX_BY_SMALL) ? 5 : 1)
 // a row of a slot plane: 33 doubles, so that lanes in successive rows hit
 // successive banks
 constexpr int FLUX_SLOT_W = 33;
-template <bool PARA, bool FFDE, int BY, bool SPLIT>
+template <bool PARA, bool FFDE, int BY, bool SPLIT, bool SP>
 __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
     k_flux_fp64(const __grid_constant__ StepArgs a, const __grid_constant__ CUtensorMap prim_map)
 {
@@ -667,7 +724,7 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
   // blocks: 1024^2 298 -> 291 us; the small grids of 4-row ones keep their
   // metric in L2, and their steps were 2% slower with it)
   FaceGeo g;
-  if (BY == FLUX_BY_LARGE) load_face_geo(a, does1 ? 1 : 2, z, g);
+  if (BY == FLUX_BY_LARGE) load_face_geo<SP>(a, does1 ? 1 : 2, z, g);
   __syncthreads();  // the barrier is initialised before anyone polls it
   if (!mbar_wait(&bar, 0)) {
     if (tx == 0 && ty == 0) report_fail(a.sc, a.phase0 + PH_FACE1, FAIL_TMA_TIMEOUT, zone_order(i, j));
@@ -734,9 +791,9 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
       if (!todo) continue;
       const double* left = slot + (2 * dir - 2) * NPR * KS;
       double Fx[NX], dtij;
-      if ((dir == 2 && does1) || BY != FLUX_BY_LARGE) load_face_geo(a, dir, z, g);
+      if ((dir == 2 && does1) || BY != FLUX_BY_LARGE) load_face_geo<SP>(a, dir, z, g);
       auto ex = ex0;
-      face_flux_x<FFDE>(ex, a, g, dir, left, left + NPR * KS, KS, Fx, dtij, rf);
+      face_flux_x<FFDE, SP>(ex, a, g, dir, left, left + NPR * KS, KS, Fx, dtij, rf);
       if (ex.ok()) {
         store_face_x(a, i, j, dir, z, Fx);
         if (dir == 1) dt1 = (dtij < dt1) ? dtij : dt1;
@@ -745,8 +802,10 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
       }
     }
   };
-  if (!tiny) faces(Exact());
-  else faces(ExactTiny());
+  if (!SP || __ldg(a.geo_full) == 0) {  // (a geometry uploaded since the kernel was chosen)
+    if (!tiny) faces(Exact());
+    else faces(ExactTiny());
+  }
 #pragma unroll 1
   for (int dir = 1; dir <= 2; dir++) {
     if (!((dir == 1) ? todo1 : todo2)) continue;
@@ -757,9 +816,9 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
   flux_block_dt(a, dt1, dt2, sh);
 }
 
-// the k_flux instance of the block's row count (b.y); its dynamic shared
-// memory limit raised once to its size
-template <typename T, bool PARA, bool FFDE, int BY>
+// the k_flux instance of the block's row count (b.y) and the metric's form;
+// its dynamic shared memory limit raised once to its size
+template <typename T, bool PARA, bool FFDE, int BY, bool SP>
 inline void flux_launch_by(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map)
 {
   constexpr bool fp64 = sizeof(T) == 8;
@@ -771,8 +830,8 @@ inline void flux_launch_by(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, co
   // -> 75.2, 245 x 131 90.9 -> 86.2 (the next size up fills the SMs anyway).
   constexpr bool small = fp64 && BY == FLUX_BY_SMALL;
   if (small && g.x * g.y <= 2 * 148) g.z = 2;
-  if constexpr (small) kern = (g.z == 2) ? k_flux_fp64<PARA, FFDE, BY, true> : k_flux_fp64<PARA, FFDE, BY, false>;
-  else if constexpr (fp64) kern = k_flux_fp64<PARA, FFDE, BY, false>;
+  if constexpr (small) kern = (g.z == 2) ? k_flux_fp64<PARA, FFDE, BY, true, SP> : k_flux_fp64<PARA, FFDE, BY, false, SP>;
+  else if constexpr (fp64) kern = k_flux_fp64<PARA, FFDE, BY, false, SP>;
   else kern = k_flux<T, PARA, FFDE, BY>;
   static bool attr[2] = {false, false};
   if (!attr[g.z - 1]) {
@@ -781,11 +840,11 @@ inline void flux_launch_by(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, co
   }
   kern<<<g, b, sm, s>>>(a, map);
 }
-template <typename T, bool PARA, bool FFDE>
+template <typename T, bool PARA, bool FFDE, bool SP>
 inline void flux_rows_launch(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map)
 {
-  if (b.y == FLUX_BY_LARGE) flux_launch_by<T, PARA, FFDE, FLUX_BY_LARGE>(g, b, s, a, map);
-  else flux_launch_by<T, PARA, FFDE, FLUX_BY_SMALL>(g, b, s, a, map);
+  if (b.y == FLUX_BY_LARGE) flux_launch_by<T, PARA, FFDE, FLUX_BY_LARGE, SP>(g, b, s, a, map);
+  else flux_launch_by<T, PARA, FFDE, FLUX_BY_SMALL, SP>(g, b, s, a, map);
 }
 
 // flux_ct corner EMF, step_ch.c:1214-1234, over i in [0,N1], j in [0,N2].
@@ -948,6 +1007,7 @@ __device__ __forceinline__ int newton_vsq_x(ExactTiny& ex, const U2PCtx& c, doub
 }
 
 // c, gn: the packed g_{mu nu} and g^{mu nu}; sg: sqrt(-g)
+template <bool SP>
 __device__ __forceinline__ int utoprim_2d_x(ExactTiny& ex, const double* U, const double* c, const double* gn, double sg,
                                             double* pr, double gam, double gammafail, int* niter, int maxit, double* nst,
                                             long long nss, bool resume)
@@ -975,11 +1035,11 @@ __device__ __forceinline__ int utoprim_2d_x(ExactTiny& ex, const double* U, cons
   const double* Q = Ut + UU;
   U2PCtx x;
   x.gam = gam;
-  const double Bv1 = c[4] * B[0] + c[5] * B[1] + c[6] * B[2], Bv2 = c[5] * B[0] + c[7] * B[1] + c[8] * B[2];
-  const double Bv3 = c[6] * B[0] + c[8] * B[1] + c[9] * B[2];
-  x.Bsq = B[0] * Bv1 + B[1] * Bv2 + B[2] * Bv3;
+  double Bv[3];
+  lower_space<SP>(B, c, Bv);
+  x.Bsq = B[0] * Bv[0] + B[1] * Bv[1] + B[2] * Bv[2];
   double Qcon[4];
-  lower_v(Q, gn, Qcon);
+  raise_con<SP>(Q, gn, Qcon);
   const double QdotB = Q[1] * B[0] + Q[2] * B[1] + Q[3] * B[2];
   x.QdotBsq = QdotB * QdotB;
   const double nlapse = -ex.sqrt_of(Exact::quot(1., ex.rcp(ngn)));
@@ -991,6 +1051,7 @@ __device__ __forceinline__ int utoprim_2d_x(ExactTiny& ex, const double* U, cons
   for (int i = 1; i < 4; i++)
 #pragma unroll
     for (int j = 1; j < 4; j++) {
+      if (SP && (SP_COV >> sym(i, j) & 1)) continue;
       const double t = c[sym(i, j)] * pr[U1 + i - 1] * pr[U1 + j - 1];
       utsq = (i == 1 && j == 1) ? t : utsq + t;
     }
@@ -1029,7 +1090,7 @@ __device__ __forceinline__ int utoprim_2d_x(ExactTiny& ex, const double* U, cons
   const Recip r1 = ex.rcp(WB), r2 = ex.rcp(W * WB);
 #pragma unroll
   for (int i = 1; i < 4; i++) {
-    const double Qt = Qcon[i] + (gn[i] * nlapse) * x.Qdotn;
+    const double Qt = (SP && i > 1) ? Qcon[i] : Qcon[i] + (gn[i] * nlapse) * x.Qdotn;
     const double t1 = ex.Exact::div(-gamma * Qt, r1), n2 = gamma * QdotB * B[i - 1];
     // the field's part is watched only where the other does not drown it
     ex.numerator((fabs(t1) > 1.e-150) ? 0. : n2);
@@ -1039,6 +1100,7 @@ __device__ __forceinline__ int utoprim_2d_x(ExactTiny& ex, const double* U, cons
 }
 
 // utoprim_ffde and fixup1zone's Lorentz limit the same way
+template <bool SP>
 __device__ __forceinline__ void utoprim_ffde_x(ExactTiny& ex, const double* U, const double* c, const double* gn,
                                                double sg, double* pr, double gammamax)
 {
@@ -1050,31 +1112,32 @@ __device__ __forceinline__ void utoprim_ffde_x(ExactTiny& ex, const double* U, c
     B[k] = ex.div(U[B1 + k], rs);
   }
   const double alphasq = Exact::quot(1., ex.rcp(-gn[0]));
-  const double b1 = c[4] * B[0] + c[5] * B[1] + c[6] * B[2], b2 = c[5] * B[0] + c[7] * B[1] + c[8] * B[2];
-  const double b3 = c[6] * B[0] + c[8] * B[1] + c[9] * B[2];
+  double bv[3];
+  lower_space<SP>(B, c, bv);
+  const double b1 = bv[0], b2 = bv[1], b3 = bv[2];
   const double Bsq = b1 * B[0] + b2 * B[1] + b3 * B[2];
   const double o = Exact::quot(1., ex.rcp(Bsq * sg));
-  const double E1 = (b2 * S[2] - b3 * S[1]) * o, E2 = (b3 * S[0] - b1 * S[2]) * o, E3 = (b1 * S[1] - b2 * S[0]) * o;
-  const double e1 = c[4] * E1 + c[5] * E2 + c[6] * E3, e2 = c[5] * E1 + c[7] * E2 + c[8] * E3;
-  const double e3 = c[6] * E1 + c[8] * E2 + c[9] * E3;
-  const double Esq = E1 * e1 + E2 * e2 + E3 * e3;
+  const double E[3] = {(b2 * S[2] - b3 * S[1]) * o, (b3 * S[0] - b1 * S[2]) * o, (b1 * S[1] - b2 * S[0]) * o};
+  double ev[3];
+  lower_space<SP>(E, c, ev);
+  const double e1 = ev[0], e2 = ev[1], e3 = ev[2];
+  const double Esq = E[0] * e1 + E[1] * e2 + E[2] * e3;
   const double gammasq = ex.Exact::div(Bsq, ex.rcp(Bsq - Esq));
   ex.need(gammasq <= gammamax * gammamax && gammasq >= 1.0);
   double v[4], uc[4];
   v[1] = alphasq * (-gn[1] + (e2 * b3 - e3 * b2) * o);
-  v[2] = alphasq * (-gn[2] + (e3 * b1 - e1 * b3) * o);
-  v[3] = alphasq * (-gn[3] + (e1 * b2 - e2 * b1) * o);
-  const double discr = +c[0] + c[4] * v[1] * v[1] + c[7] * v[2] * v[2] + c[9] * v[3] * v[3] +
-                       2. * (c[1] * v[1] + c[2] * v[2] + c[3] * v[3] + c[5] * v[1] * v[2] + c[6] * v[1] * v[3] +
-                             c[8] * v[2] * v[3]);
+  v[2] = alphasq * (SP ? (e3 * b1 - e1 * b3) * o : -gn[2] + (e3 * b1 - e1 * b3) * o);
+  v[3] = alphasq * (SP ? (e1 * b2 - e2 * b1) * o : -gn[3] + (e1 * b2 - e2 * b1) * o);
+  const double d2 = SP ? c[1] * v[1] + c[3] * v[3] + c[6] * v[1] * v[3]
+                       : c[1] * v[1] + c[2] * v[2] + c[3] * v[3] + c[5] * v[1] * v[2] + c[6] * v[1] * v[3] +
+                             c[8] * v[2] * v[3];
+  const double discr = +c[0] + c[4] * v[1] * v[1] + c[7] * v[2] * v[2] + c[9] * v[3] * v[3] + 2. * d2;
   uc[0] = Exact::quot(1., ex.rcp(ex.sqrt_of(-discr)));
 #pragma unroll
   for (int j = 1; j < 4; j++) pr[U1 - 1 + j] = v[j] * uc[0];
 #pragma unroll
   for (int k = 0; k < 3; k++) pr[B1 + k] = B[k];
-  const double qsq = c[4] * pr[U1] * pr[U1] + c[7] * pr[U2] * pr[U2] + c[9] * pr[U3] * pr[U3] +
-                     2. * (c[5] * pr[U1] * pr[U2] + c[6] * pr[U1] * pr[U3] + c[8] * pr[U2] * pr[U3]);
-  ex.need(gammamax <= 1.0 || ex.sqrt_of(1. + qsq) <= gammamax);
+  ex.need(gammamax <= 1.0 || ex.sqrt_of(1. + qsq_x<SP>(pr, c)) <= gammamax);
 }
 
 // flux divergence with flux-CT B fluxes (step_ch.c:1403-1413)
@@ -1216,7 +1279,7 @@ __device__ __noinline__ int update_general(const StepArgs& a, int i, int j, cons
 // us with the tail at 512^2).  A zone whose values leave the exact range goes
 // to update_general.  512^2 developed flow: 86 -> 50 us (first substep) and
 // 58 us (second), 3.9 TB/s; 1024^2 with the tail 300 -> 178 us.
-template <typename FT, bool FFDE>
+template <typename FT, bool FFDE, bool SP>
 __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepArgs a,
                                                    const __grid_constant__ CUtensorMap geo_map,
                                                    const double* __restrict__ pi, const double* __restrict__ pb,
@@ -1254,9 +1317,10 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
   {
     const double* base = a.geo + (long long)CENT * GEO_PER_LOC * pl + z;
 #pragma unroll
-    for (int k = 0; k < 10; k++) c[k] = __ldg(base + k * pl);
-#pragma unroll
-    for (int k = 0; k < 10; k++) gn[k] = __ldg(base + (10 + k) * pl);
+    for (int k = 0; k < 10; k++) {
+      if (!SP || !(SP_COV >> k & 1)) c[k] = __ldg(base + k * pl);
+      if (!SP || !(SP_CON >> k & 1)) gn[k] = __ldg(base + (10 + k) * pl);
+    }
     sg = __ldg(base + 20 * pl);
 #pragma unroll
     for (int k = 0; k < NPR; k++) pfz[k] = __ldg(pi + k * pl + z);
@@ -1267,8 +1331,9 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
   for (int k = 0; k < NPR; k++) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(prb[k]) : "l"(pb + k * pl + z));
   __syncthreads();  // the barrier is initialised before anyone polls it
   if (active) {
-    lp = lapse_x(ex, gn);
-    state_x(ex, pfz, c, lp, 1.e300, q);
+    if (SP) ex.need(__ldg(a.geo_full) == 0);  // (a geometry uploaded since the kernel was chosen)
+    lp = lapse_x<SP>(ex, gn);
+    state_x<SP>(ex, pfz, c, lp, 1.e300, q);
     // Ui = U(pi)
     conserved_x<FFDE>(pfz, q, sg, gam, U);
     if (a.bsqf_fused) bf = bsq_flag_x(ex, a, pfz, q.bsq);  // get_bsqflags of the step's p
@@ -1282,7 +1347,7 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
   const double* sz = sgeo + threadIdx.y * W + threadIdx.x + 1;
   {
     // (the first substep's pb is pi, whose state is at hand)
-    if (pb != pi) state_x(ex, prb, c, lp, 1.e300, q);
+    if (pb != pi) state_x<SP>(ex, prb, c, lp, 1.e300, q);
     const double r = FFDE ? 0. : prb[RHO], u = FFDE ? 0. : prb[UU], P = (gam - 1.) * u, w = P + r + u;
     const double eta = FFDE ? q.bsq : w + q.bsq, ptot = FFDE ? q.bsq * 0.5 : P + q.bsq * 0.5;
     double acc[4] = {0., 0., 0., 0.};
@@ -1307,7 +1372,7 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
     }
   }
   if constexpr (FFDE) {
-    utoprim_ffde_x(ex, U, c, gn, sg, pfz, a.pp.gammamax);
+    utoprim_ffde_x<SP>(ex, U, c, gn, sg, pfz, a.pp.gammamax);
     if (!ex.ok()) {
       update_general<FT, FFDE>(a, i, j, pi, pb, pf, c2, sz, plane_s);
       return;
@@ -1318,7 +1383,7 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
     int niter;
     // a deferred solve leaves its Newton state in the repair scratch (idle
     // until k_fixup_compute), NEWTON_STATE planes
-    const int pfl = utoprim_2d_x(ex, U, c, gn, sg, pfz, gam, a.pp.gammafail, &niter, NEWTON_MAIN_CAP, a.fixbuf + z, pl,
+    const int pfl = utoprim_2d_x<SP>(ex, U, c, gn, sg, pfz, gam, a.pp.gammafail, &niter, NEWTON_MAIN_CAP, a.fixbuf + z, pl,
                                  false);
     if (!ex.ok()) {
       niter = update_general<FT, FFDE>(a, i, j, pi, pb, pf, c2, sz, plane_s);
@@ -1330,7 +1395,7 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
       } else {
         Geo<double> g;
 #pragma unroll
-        for (int k = 0; k < 10; k++) g.gcov[k] = c[k];
+        for (int k = 0; k < 10; k++) g.gcov[k] = (SP && (SP_COV >> k & 1)) ? 0. : c[k];
         finish_zone(a, g, z, i, j, pfz, pfl, pf, sz[(GEO_FLOOR - GEO_CONN) * plane_s],
                     sz[(GEO_FLOOR + 1 - GEO_CONN) * plane_s]);
       }
@@ -1345,9 +1410,9 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
 // launches a k_update instance (its dynamic shared memory limit raised once
 // to the largest box of the tile shapes harm_set_tiles accepts: 42 planes x
 // at most 128 threads)
-template <typename FT, bool FFDE>
-inline void update_launch(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map, const double* pi,
-                          const double* pb, double* pf, double c2)
+template <typename FT, bool FFDE, bool SP>
+inline void update_launch_sp(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map, const double* pi,
+                             const double* pb, double* pf, double c2)
 {
   static bool attr = false;
   if (!attr) {
@@ -1357,10 +1422,17 @@ inline void update_launch(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, con
       const size_t v = upd_smem_bytes(bx + (bx & 1), by);
       if (v > mx) mx = v;
     }
-    cudaFuncSetAttribute(k_update<FT, FFDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx);
+    cudaFuncSetAttribute(k_update<FT, FFDE, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx);
     attr = true;
   }
-  k_update<FT, FFDE><<<g, b, upd_smem_bytes(b.x, b.y), s>>>(a, map, pi, pb, pf, c2);
+  k_update<FT, FFDE, SP><<<g, b, upd_smem_bytes(b.x, b.y), s>>>(a, map, pi, pb, pf, c2);
+}
+template <typename FT, bool FFDE>
+inline void update_launch(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map, const double* pi,
+                          const double* pb, double* pf, double c2)
+{
+  if (a.sparse) update_launch_sp<FT, FFDE, true>(g, b, s, a, map, pi, pb, pf, c2);
+  else update_launch_sp<FT, FFDE, false>(g, b, s, a, map, pi, pb, pf, c2);
 }
 
 // ---------------------------------------------------------------- end of step

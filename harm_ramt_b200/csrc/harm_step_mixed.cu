@@ -12,10 +12,10 @@ void launch_flux_mixed(int para, int ffde, dim3 g, dim3 b, cudaStream_t s, const
                        const CUtensorMap& prim_map)
 {
   if (ffde) {
-    if (para) flux_rows_launch<float, true, true>(g, b, s, a, prim_map);
-    else flux_rows_launch<float, false, true>(g, b, s, a, prim_map);
-  } else if (para) flux_rows_launch<float, true, false>(g, b, s, a, prim_map);
-  else flux_rows_launch<float, false, false>(g, b, s, a, prim_map);
+    if (para) flux_rows_launch<float, true, true, false>(g, b, s, a, prim_map);
+    else flux_rows_launch<float, false, true, false>(g, b, s, a, prim_map);
+  } else if (para) flux_rows_launch<float, true, false, false>(g, b, s, a, prim_map);
+  else flux_rows_launch<float, false, false, false>(g, b, s, a, prim_map);
 }
 
 void launch_emf_mixed(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const double* pv)
