@@ -82,6 +82,7 @@ struct harm_ctx {
   int flux_by;       // k_flux rows per block (flux_rows)
   bool geo_ok;
   int sparse;        // the uploaded metric is of the sparse form (SP in harm_step_impl.cuh)
+  bool in_ensemble;  // captured into an ensemble's graph, which outlives an upload
   cudaGraph_t graph;
   cudaGraphExec_t gexec;
   bool have_graph;
@@ -112,6 +113,7 @@ struct harm_ctx {
     a.geo = d_geo;
     a.geo32 = d_geo32;
     a.sparse = sparse;
+    a.sparse32 = sparse && !in_ensemble;
     a.geo_full = reinterpret_cast<const int*>(d_geo + GEO_NPLANES * gr.plane);
     a.F1 = d_F1;
     a.F2 = d_F2;
@@ -937,6 +939,7 @@ int harm_ensemble_create(harm_ctx* const* members, int n, int per_launch, void* 
       cap_ok = cudaStreamWaitEvent(br[k], ev[n], 0) == cudaSuccess;
       harm_ctx tmp = *e->m[k];
       tmp.stream = br[k];
+      tmp.in_ensemble = true;
       for (int sidx = 0; sidx < per_launch && cap_ok; sidx++) cap_ok = enqueue_step(&tmp) == HARM_OK;
       if (cap_ok) cap_ok = cudaEventRecord(ev[k], br[k]) == cudaSuccess;
       if (cap_ok) cap_ok = cudaStreamWaitEvent(e->stream, ev[k], 0) == cudaSuccess;

@@ -62,25 +62,33 @@ struct State {
 template <typename T>
 HD_INLINE T pick4(const T* v, int d) { return (d == 3) ? v[3] : ((d == 2) ? v[2] : ((d == 1) ? v[1] : v[0])); }
 
+// SP (gamma_of to vchar_of): a metric with g_{t2} = g_{12} = g_{23} = 0 and
+// g^{t2} = g^{t3} = 0, whose products are left out (they are exact zeros, so
+// for finite values the sums stay the same; ucon_of keeps its shift terms:
+// without them the compiler contracts the FP32 faces' sums differently, which
+// moved the mixed form by 1e-7)
 // gamma_calc, phys.c:848-877
-template <typename T>
+template <typename T, bool SP = false>
 HD_INLINE T gamma_of(const T* pr, const Geo<T>& g)
 {
   const T* c = g.gcov;
+  if (SP)
+    return sqrt(T(1.) + (c[4] * pr[U1] * pr[U1] + c[7] * pr[U2] * pr[U2] + c[9] * pr[U3] * pr[U3] +
+                         T(2.) * (c[6] * pr[U1] * pr[U3])));
   T qsq = c[4] * pr[U1] * pr[U1] + c[7] * pr[U2] * pr[U2] + c[9] * pr[U3] * pr[U3] +
           T(2.) * (c[5] * pr[U1] * pr[U2] + c[6] * pr[U1] * pr[U3] + c[8] * pr[U2] * pr[U3]);
   return sqrt(T(1.) + qsq);
 }
 
 // ucon_calc_rel4vel, phys.c:830-845
-template <typename T>
+template <typename T, bool SP = false>
 HD_INLINE void ucon_of(const T* pr, const Geo<T>& g, T* ucon)
 {
   T alpha = T(1.) / sqrt(-g.gcon[0]);
   T beta1 = g.gcon[1] * alpha * alpha;
   T beta2 = g.gcon[2] * alpha * alpha;
   T beta3 = g.gcon[3] * alpha * alpha;
-  T gamma = gamma_of(pr, g);
+  T gamma = gamma_of<T, SP>(pr, g);
   ucon[0] = gamma / alpha;
   ucon[1] = pr[U1] - gamma * beta1 / alpha;
   ucon[2] = pr[U2] - gamma * beta2 / alpha;
@@ -88,9 +96,16 @@ HD_INLINE void ucon_of(const T* pr, const Geo<T>& g, T* ucon)
 }
 
 // lower, phys.c:633
-template <typename T>
+template <typename T, bool SP = false>
 HD_INLINE void lower_v(const T* v, const T* c, T* w)
 {
+  if (SP) {
+    w[0] = c[0] * v[0] + c[1] * v[1] + c[3] * v[3];
+    w[1] = c[1] * v[0] + c[4] * v[1] + c[6] * v[3];
+    w[2] = c[7] * v[2];
+    w[3] = c[3] * v[0] + c[6] * v[1] + c[9] * v[3];
+    return;
+  }
   w[0] = c[0] * v[0] + c[1] * v[1] + c[2] * v[2] + c[3] * v[3];
   w[1] = c[1] * v[0] + c[4] * v[1] + c[5] * v[2] + c[6] * v[3];
   w[2] = c[2] * v[0] + c[5] * v[1] + c[7] * v[2] + c[8] * v[3];
@@ -101,15 +116,15 @@ template <typename T>
 HD_INLINE T dot4(const T* a, const T* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2] + a[3] * b[3]; }
 
 // get_state + bcon_calc, phys.c:716-727 and 285-294
-template <typename T>
+template <typename T, bool SP = false>
 HD_INLINE void state_of(const T* pr, const Geo<T>& g, State<T>& q)
 {
-  ucon_of(pr, g, q.ucon);
-  lower_v(q.ucon, g.gcov, q.ucov);
+  ucon_of<T, SP>(pr, g, q.ucon);
+  lower_v<T, SP>(q.ucon, g.gcov, q.ucov);
   q.bcon[0] = pr[B1] * q.ucov[1] + pr[B2] * q.ucov[2] + pr[B3] * q.ucov[3];
 #pragma unroll
   for (int j = 1; j <= 3; j++) q.bcon[j] = (pr[B1 - 1 + j] + q.bcon[0] * q.ucon[j]) / q.ucon[0];
-  lower_v(q.bcon, g.gcov, q.bcov);
+  lower_v<T, SP>(q.bcon, g.gcov, q.bcov);
 }
 
 // mhd_calc_0, phys.c:381-406 (row `dir` of T^mu_nu)
@@ -160,7 +175,7 @@ HD_INLINE void flux_of(const T* pr, const State<T>& q, int dir, const Geo<T>& g,
 // vchar + simplefast, vchar.c:37-135 and 166-234.  The raised unit covectors
 // reduce to metric columns, so the dot products are the metric entries the
 // reference's zero-padded sums produce.  Returns a fail code.
-template <typename T>
+template <typename T, bool SP = false>
 HD_INLINE int vchar_of(const T* pr, const State<T>& q, int dir, const Geo<T>& g, T gam, T& vmax, T& vmin)
 {
   // NUMEPSILON*100 of the reference's FTYPE (global.h:706-727): DBL_EPSILON
@@ -198,6 +213,14 @@ HD_INLINE int vchar_of(const T* pr, const State<T>& q, int dir, const Geo<T>& g,
   T Au = T(dir == 0) * q.ucon[0] + T(dir == 1) * q.ucon[1] + T(dir == 2) * q.ucon[2] + T(dir == 3) * q.ucon[3];
   T Bu = T(1.) * q.ucon[0] + T(0.) * q.ucon[1] + T(0.) * q.ucon[2] + T(0.) * q.ucon[3];
   T AB = Acon[0] * T(1.) + Acon[1] * T(0.) + Acon[2] * T(0.) + Acon[3] * T(0.);
+  if (SP) {
+    // (dir is 1 or 2) the same without the zero terms
+    Asq = (dir == 1) ? g.gcon[4] : g.gcon[7];
+    Bsq = g.gcon[0];
+    Au = (dir == 1) ? q.ucon[1] : q.ucon[2];
+    Bu = q.ucon[0];
+    AB = (dir == 1) ? g.gcon[1] : T(0.);
+  }
   T Au2 = Au * Au, Bu2 = Bu * Bu, AuBu = Au * Bu;
   T A = Bu2 - (Bsq + Bu2) * cms2;
   T B = T(2.) * (AuBu - (AB + AuBu) * cms2);
@@ -223,11 +246,11 @@ HD_INLINE int vchar_of(const T* pr, const State<T>& q, int dir, const Geo<T>& g,
 }
 
 // limit_gamma, fixup.c:1298-1354.  Returns a fail code.
-template <typename T>
+template <typename T, bool SP = false>
 HD_INLINE int limit_gamma(T gammamax, T* pr, const Geo<T>& g)
 {
   if (gammamax <= T(1.0)) return 0;
-  T gamma = gamma_of(pr, g);
+  T gamma = gamma_of<T, SP>(pr, g);
   if (gamma > gammamax && gamma != T(1.0)) {
     T pref = (gammamax * gammamax - T(1.)) / (gamma * gamma - T(1.));
     if (pref < T(0.0)) return FAIL_UTCALC_DISCR;

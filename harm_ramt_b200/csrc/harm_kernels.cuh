@@ -81,6 +81,7 @@ struct StepArgs {
   const double* geo;     // GEO_NPLANES planes
   const int* geo_full;   // nonzero: the uploaded metric is not of the sparse form
   int sparse;            // kernels for the sparse form (SP in harm_step_impl.cuh) are chosen
+  int sparse32;          // the same for the FP32 faces, which do not look at geo_full
   const float* geo32;    // mixed precision: FACE1 and FACE2 geometry (2 x 21 float planes)
   double* F1;            // 8 planes (of float in mixed precision)
   double* F2;            // 8 planes (of float in mixed precision)
@@ -149,14 +150,19 @@ __device__ __forceinline__ void report_fail(DevScalars* sc, int phase, int code,
   atomicMax(&sc->fail_inv, ~fail_key(sc->realnstep, phase, order, code));
 }
 
-// FP32 copy of a face location's geometry (mixed precision)
+// FP32 copy of a face location's geometry (mixed precision; SP: the entries
+// that the sparse form does not use are not set)
+template <bool SP>
 __device__ __forceinline__ void load_geo32(const StepArgs& a, int loc, long long z, Geo<float>& g)
 {
   const float* base = a.geo32 + (long long)loc * GEO_PER_LOC * a.gr.plane + z;
 #pragma unroll
-  for (int c = 0; c < 10; c++) g.gcov[c] = __ldg(base + c * a.gr.plane);
+  for (int c = 0; c < 10; c++)
+    if (!SP || (c != 2 && c != 5 && c != 8)) g.gcov[c] = __ldg(base + c * a.gr.plane);
 #pragma unroll
-  for (int c = 0; c < 10; c++) g.gcon[c] = __ldg(base + (10 + c) * a.gr.plane);
+  for (int c = 0; c < 10; c++)
+    if (!SP || (c != 2 && c != 3 && c != 5 && c != 8)) g.gcon[c] = __ldg(base + (10 + c) * a.gr.plane);
+  if (SP) g.gcon[2] = g.gcon[3] = 0.f;
   g.g = __ldg(base + 20 * a.gr.plane);
 }
 

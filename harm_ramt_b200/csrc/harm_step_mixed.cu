@@ -8,14 +8,21 @@
 
 namespace harm {
 
+template <bool SP>
+static void flux_fp32(int para, int ffde, dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& prim_map)
+{
+  if (ffde) {
+    if (para) flux_rows_launch<float, true, true, SP>(g, b, s, a, prim_map);
+    else flux_rows_launch<float, false, true, SP>(g, b, s, a, prim_map);
+  } else if (para) flux_rows_launch<float, true, false, SP>(g, b, s, a, prim_map);
+  else flux_rows_launch<float, false, false, SP>(g, b, s, a, prim_map);
+}
+
 void launch_flux_mixed(int para, int ffde, dim3 g, dim3 b, cudaStream_t s, const StepArgs& a,
                        const CUtensorMap& prim_map)
 {
-  if (ffde) {
-    if (para) flux_rows_launch<float, true, true, false>(g, b, s, a, prim_map);
-    else flux_rows_launch<float, false, true, false>(g, b, s, a, prim_map);
-  } else if (para) flux_rows_launch<float, true, false, false>(g, b, s, a, prim_map);
-  else flux_rows_launch<float, false, false, false>(g, b, s, a, prim_map);
+  if (a.sparse32) flux_fp32<true>(para, ffde, g, b, s, a, prim_map);
+  else flux_fp32<false>(para, ffde, g, b, s, a, prim_map);
 }
 
 void launch_emf_mixed(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const double* pv)

@@ -76,3 +76,22 @@ def test_ensemble_member_changes_form(harm):
     for h, g in zip(m, (sparse, full)):
         assert np.array_equal(h.get_prims()[0], _oracle(g, p0, 4, 1, 4)[0])
     e.close()
+
+
+def test_mixed_forms_agree(harm):
+    """An ensemble's FP32 faces use the form for any metric, a context's own
+    step the sparse one: the same bits."""
+    par = harm.torus_params(N1, N2)
+    g = harm.torus_geometry(par)
+    p0 = harm.torus_init(par, g)
+    m = [harm.HarmGPU(N1, N2, g["dx1"], g["dx2"], lim=4, fluxmethod=1, precision=harm.PREC_MIXED) for _ in range(2)]
+    for h in m:
+        _upload(h, g)
+        _start(h, p0)
+    e = harm.Ensemble(m[:1], steps_per_launch=3)
+    e.step(30)
+    e.sync()
+    m[1].step_ch(30)
+    m[1].sync()
+    assert np.array_equal(m[0].get_prims()[0], m[1].get_prims()[0])
+    e.close()
