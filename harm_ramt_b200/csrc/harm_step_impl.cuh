@@ -11,70 +11,46 @@
 namespace harm {
 
 // ---------------------------------------------------------------- fluxes
-// Interface states of a zone along `dir` (step_ch.c:812-823 slopes and
-// 893-904 interface values) from its stencil in the block's primitive tile
-// (shared memory): L = the zone's left-face value (p_r of face i), R = its
-// right-face value (p_l of face i+1).  t points at the zone's value of
-// plane 0; planes are `ps` doubles apart, the stencil step is `st` (1 along
-// x1, the tile width along x2).
-template <typename T, bool PARA>
-__device__ __forceinline__ void zone_states(const double* t, int ps, int st, T* L, T* R)
-{
-#pragma unroll
-  for (int k = 0; k < NPR; k++) {
-    const double* pk = t + k * ps;
-    if (!PARA) {
-      T ym1 = (T)pk[-st], y0 = (T)pk[0], yp1 = (T)pk[st];
-      T dq = mc_slope(ym1, y0, yp1);
-      L[k] = y0 - T(0.5) * dq;
-      R[k] = y0 + T(0.5) * dq;
-    } else {
-      T l, r;
-      para4((T)pk[-2 * st], (T)pk[-st], (T)pk[0], (T)pk[st], (T)pk[2 * st], l, r);
-      L[k] = l;
-      R[k] = r;
-    }
-  }
-}
-
-// The FP64 interface states of N consecutive zones of one variable, a thread
+// The interface states (step_ch.c:812-823 slopes and 893-904 interface
+// values) of N consecutive zones of one variable, a thread
 // walking along the zones (src: the first zone's value, step st; one more
 // value on each side is read for MC, two for PARA).  The slopes and, for
 // PARA, the raw interface values that neighbouring zones share are formed
 // once; put(c, l, r) takes zone c's states.  The values are mc_slope's and
 // para4's: 2 min(|a|, |b|) is min(|2 a|, |2 b|), (4 a) b is (2 a)(2 b), and
 // the sign of a slope is copied instead of multiplied.
-__device__ __forceinline__ double para_dq_shared(double a, double b, double ym, double yp)
+template <typename T>
+__device__ __forceinline__ T para_dq_shared(T a, T b, T ym, T yp)
 {
-  const double s = (4. * a) * b, c = 0.5 * (yp - ym);
-  const double m = 2. * rmin(fabs(a), fabs(b));
-  return (s <= 0.) ? 0. : copysign(rmin(fabs(c), m), c);
+  const T s = (T(4.) * a) * b, c = T(0.5) * (yp - ym);
+  const T m = T(2.) * rmin(fabs(a), fabs(b));
+  return (s <= T(0.)) ? T(0.) : copysign(rmin(fabs(c), m), c);
 }
-template <bool PARA, int N, typename Put>
+template <typename T, bool PARA, int N, typename Put>
 __device__ __forceinline__ void row_states(const double* src, int st, Put put)
 {
-  double ym = src[-st], y = src[0], a = y - ym;
+  T ym = (T)src[-st], y = (T)src[0], a = y - ym;
   if (!PARA) {
 #pragma unroll
     for (int c = 0; c < N; c++) {
-      const double yp = src[(c + 1) * st], b = yp - y;
-      const double h = 0.5 * minmod(0.5 * (yp - ym), minmod(2. * a, 2. * b));
+      const T yp = (T)src[(c + 1) * st], b = yp - y;
+      const T h = T(0.5) * minmod(T(0.5) * (yp - ym), minmod(T(2.) * a, T(2.) * b));
       put(c, y - h, y + h);
       ym = y;
       y = yp;
       a = b;
     }
   } else {
-    double yp = src[st], b = yp - y;
-    const double ymm = src[-2 * st];
-    double d0 = para_dq_shared(ym - ymm, a, ymm, y), d = para_dq_shared(a, b, ym, yp);
-    double l = para_face(ym, y, d0, d);
+    T yp = (T)src[st], b = yp - y;
+    const T ymm = (T)src[-2 * st];
+    T d0 = para_dq_shared(ym - ymm, a, ymm, y), d = para_dq_shared(a, b, ym, yp);
+    T l = para_face(ym, y, d0, d);
 #pragma unroll
     for (int c = 0; c < N; c++) {
-      const double ypp = src[(c + 2) * st], e = ypp - yp;
-      const double d1 = para_dq_shared(b, e, y, ypp);
-      const double r = para_face(y, yp, d, d1);
-      double lo, ro;
+      const T ypp = (T)src[(c + 2) * st], e = ypp - yp;
+      const T d1 = para_dq_shared(b, e, y, ypp);
+      const T r = para_face(y, yp, d, d1);
+      T lo, ro;
       para_limit(ym, y, yp, l, r, lo, ro);
       put(c, lo, ro);
       ym = y;
@@ -536,6 +512,42 @@ __device__ __forceinline__ const double* flux_tile_load(double* tile, const CUte
   return tile + (ty + 3) * FLUX_TILE_W + tx + 2 + ((int)(blockIdx.x * FLUX_BX) - cx);
 }
 
+// a row of a slot plane: 33 values, so that lanes in successive rows hit
+// successive banks
+constexpr int FLUX_SLOT_W = 33;
+// The interface states of the block's zones, from the tile (tz: the thread's
+// zone) into four slots a zone in shared memory: state s (0 left, 1 right) of
+// its face in direction dir is slot[(2 * dir - 2 + s) * NPR * KS + k * KS],
+// KS = BY * FLUX_SLOT_W.  A warp forms the states of one variable (BY = 8) or
+// two at all of the block's zones: along x2 a lane per column (and the zones
+// below the first row, for their right states), along x1 a lane per BY zones
+// of a row.  A zone's right state is the left state of the next zone's face.
+template <typename T, bool PARA, int BY>
+__device__ __forceinline__ void block_states(const double* tz, T* slot, bool does1 = true, bool does2 = true)
+{
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  constexpr int PS = flux_tile_rows(BY) * FLUX_TILE_W, SW = FLUX_SLOT_W, KS = BY * SW;
+#pragma unroll 1
+  for (int k = ty; k < NPR; k += BY) {
+    const double* t = tz + (k * PS - ty * FLUX_TILE_W - tx);  // the block's first zone
+    T* d = slot + (k * KS - ty * SW - tx);
+    if (does2) {
+      T* d2 = d + 2 * NPR * KS + tx;
+      row_states<T, PARA, BY + 1>(t + tx - FLUX_TILE_W, FLUX_TILE_W, [&](int c, T l, T r) {
+        if (c > 0) d2[NPR * KS + (c - 1) * SW] = l;
+        if (c < BY) d2[c * SW] = r;
+      });
+    }
+    if (!does1) continue;
+    const int row = tx % BY, c0 = (tx / BY) * BY;
+    d += row * SW + c0;
+    row_states<T, PARA, BY>(t + row * FLUX_TILE_W + c0, 1, [&](int c, T l, T r) {
+      d[NPR * KS + c] = l;
+      d[c + 1] = r;  // (the last zone's goes to the row's padding)
+    });
+  }
+}
+
 // the block's Courant minima
 __device__ __forceinline__ void flux_block_dt(const StepArgs& a, double dt1, double dt2, double (*sh)[32])
 {
@@ -597,18 +609,19 @@ static __device__ __noinline__ int flux_flags_x(const StepArgs& a, const double*
 // which halves the kernel's instruction footprint.  96 registers a thread:
 // five 4-row blocks per SM.  With the sparse metric's planes and products left
 // out a mixed step takes 276 -> 270 us at 512^2 and 94.4 -> 88.0 on the 512 x
-// 256 dipole, with the same bits.
+// 256 dipole; with PARA's states formed by block_states 270 -> 246 at 512^2;
+// all with the same bits.
 template <typename T, bool PARA, bool FFDE, int BY, bool SP>
 __global__ void __launch_bounds__(32 * BY, (BY == FLUX_BY_SMALL) ? 5 : 1)
     k_flux(StepArgs a, const __grid_constant__ CUtensorMap prim_map)
 {
   extern __shared__ __align__(128) double tile[];
   __shared__ double sh[2][32];
-  __shared__ T shr[NPR][BY][32];
   __shared__ uint64_t bar;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  constexpr int PS = flux_tile_rows(BY) * FLUX_TILE_W;
+  constexpr int PS = flux_tile_rows(BY) * FLUX_TILE_W, SW = FLUX_SLOT_W, KS = BY * SW;
   const double* tz = flux_tile_load<BY>(tile, &prim_map, &bar);
+  T* slot = reinterpret_cast<T*>(tile + NPR * PS) + ty * SW + tx;  // as in k_flux_fp64
   const int i = blockIdx.x * FLUX_BX + tx - 1;
   const int j = blockIdx.y * BY + ty - 1;
   const int n1 = a.gr.n1, n2 = a.gr.n2;
@@ -616,7 +629,7 @@ __global__ void __launch_bounds__(32 * BY, (BY == FLUX_BY_SMALL) ? 5 : 1)
   const bool own = (tx > 0) || (blockIdx.x == 0);  // lane 0 of a later block repeats a zone
   const long long z = a.gr.at(in ? i : -1, in ? j : -1);
   double dt1 = 1.e9, dt2 = 1.e9;
-  T L[NPR], R[NPR], pl[NPR];
+  T L[NPR], pl[NPR];
   T Fo[NPR];
   double dtij;
   T* F1 = reinterpret_cast<T*>(a.F1);
@@ -626,6 +639,7 @@ __global__ void __launch_bounds__(32 * BY, (BY == FLUX_BY_SMALL) ? 5 : 1)
     if (tx == 0 && ty == 0) report_fail(a.sc, a.phase0 + PH_FACE1, FAIL_TMA_TIMEOUT, zone_order(i, j));
     return;
   }
+  if constexpr (PARA) block_states<T, PARA, BY>(tz, slot);
   // the flux choice of this zone, which both of its faces use: fluxmethod,
   // or with the per-zone switch FLAGREALFLUX, formed in the first substep
   // and read back in the second
@@ -642,27 +656,46 @@ __global__ void __launch_bounds__(32 * BY, (BY == FLUX_BY_SMALL) ? 5 : 1)
       rf = (int)a.fluxf[z];
     }
   }
+  if constexpr (PARA) __syncthreads();
 #pragma unroll 1
   for (int dir = 1; dir <= 2; dir++) {
-    zone_states<T, PARA>(tz, PS, (dir == 1) ? 1 : FLUX_TILE_W, L, R);
-    bool act;
-    if (dir == 1) {
+    if constexpr (PARA) {
+      const T* left = slot + (2 * dir - 2) * NPR * KS;
 #pragma unroll
-      for (int k = 0; k < NPR; k++) pl[k] = __shfl_up_sync(0xffffffffu, R[k], 1);
-      act = in && i >= 0 && tx > 0;
-    } else {
-#pragma unroll
-      for (int k = 0; k < NPR; k++) shr[k][ty][tx] = R[k];
-      __syncthreads();
-      if (ty > 0) {
-#pragma unroll
-        for (int k = 0; k < NPR; k++) pl[k] = shr[k][ty - 1][tx];
-      } else {
-        T Lm[NPR];
-        zone_states<T, PARA>(tz - FLUX_TILE_W, PS, FLUX_TILE_W, Lm, pl);
+      for (int k = 0; k < NPR; k++) {
+        pl[k] = left[k * KS];
+        L[k] = left[(NPR + k) * KS];
       }
-      act = in && j >= 0 && own;
+    } else {
+      // MC's slopes are cheap: each thread forms its own zone's, and the left
+      // state comes by shuffle or through shared memory (the mixed 512 x 256
+      // dipole 88.2 us a step, with block_states 90.9)
+      const int st = (dir == 1) ? 1 : FLUX_TILE_W;
+      T R[NPR];
+#pragma unroll
+      for (int k = 0; k < NPR; k++)
+        row_states<T, false, 1>(tz + k * PS, st, [&](int, T l, T r) {
+          L[k] = l;
+          R[k] = r;
+        });
+      if (dir == 1) {
+#pragma unroll
+        for (int k = 0; k < NPR; k++) pl[k] = __shfl_up_sync(0xffffffffu, R[k], 1);
+      } else {
+#pragma unroll
+        for (int k = 0; k < NPR; k++) slot[k * KS] = R[k];
+        __syncthreads();
+        if (ty > 0) {
+#pragma unroll
+          for (int k = 0; k < NPR; k++) pl[k] = slot[k * KS - SW];
+        } else {
+#pragma unroll
+          for (int k = 0; k < NPR; k++)
+            row_states<T, false, 1>(tz + k * PS - st, st, [&](int, T, T r) { pl[k] = r; });
+        }
+      }
     }
+    const bool act = (dir == 1) ? (in && i >= 0 && tx > 0) : (in && j >= 0 && own);
     if (act) {
       face_flux<T, FFDE, SP>(a, i, j, dir, pl, L, Fo, dtij, rf);
       T* F;
@@ -699,9 +732,6 @@ __global__ void __launch_bounds__(32 * BY, (BY == FLUX_BY_SMALL) ? 5 : 1)
 // each quotient and root with its own branches -> this form): 512^2 PARA
 // with the switch 152 -> 88 us, 1024^2 626 -> 299 us, 128^2 MC 26 -> 16 us,
 // the force-free 512 x 256 dipole 63.5 -> 38 us.
-// a row of a slot plane: 33 doubles, so that lanes in successive rows hit
-// successive banks
-constexpr int FLUX_SLOT_W = 33;
 template <bool PARA, bool FFDE, int BY, bool SPLIT, bool SP>
 __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
     k_flux_fp64(const __grid_constant__ StepArgs a, const __grid_constant__ CUtensorMap prim_map)
@@ -732,29 +762,7 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
     if (tx == 0 && ty == 0) report_fail(a.sc, a.phase0 + PH_FACE1, FAIL_TMA_TIMEOUT, zone_order(i, j));
     return;
   }
-  // a warp forms the states of one variable (BY = 8) or two at all of the
-  // block's zones: along x2 a lane per column (and the zones below the first
-  // row, for their right states), along x1 a lane per BY zones of a row.  A
-  // zone's right state is the left state of the next zone's face.
-#pragma unroll 1
-  for (int k = ty; k < NPR; k += BY) {
-    const double* t = tz + (k * PS - ty * FLUX_TILE_W - tx);  // the block's first zone
-    double* d = slot + (k * KS - ty * SW - tx);
-    if (does2) {
-      double* d2 = d + 2 * NPR * KS + tx;
-      row_states<PARA, BY + 1>(t + tx - FLUX_TILE_W, FLUX_TILE_W, [&](int c, double l, double r) {
-        if (c > 0) d2[NPR * KS + (c - 1) * SW] = l;
-        if (c < BY) d2[c * SW] = r;
-      });
-    }
-    if (!does1) continue;
-    const int row = tx % BY, c0 = (tx / BY) * BY;
-    d += row * SW + c0;
-    row_states<PARA, BY>(t + row * FLUX_TILE_W + c0, 1, [&](int c, double l, double r) {
-      d[NPR * KS + c] = l;
-      d[c + 1] = r;  // (the last zone's goes to the row's padding)
-    });
-  }
+  block_states<double, PARA, BY>(tz, slot, does1, does2);
   // the flux choice of this zone (as in k_flux)
   int rf = a.pp.fluxmethod;
   if (a.pp.fluxadjust && in) {
@@ -824,7 +832,9 @@ template <typename T, bool PARA, bool FFDE, int BY, bool SP>
 inline void flux_launch_by(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map)
 {
   constexpr bool fp64 = sizeof(T) == 8;
-  constexpr size_t sm = flux_tile_bytes(BY) + (fp64 ? 4 * NPR * BY * FLUX_SLOT_W * sizeof(double) : 0);
+  // (MC's FP32 faces pass one state on: the rest of the SM's memory is L1)
+  constexpr int slots = (fp64 || PARA) ? 4 : 1;
+  constexpr size_t sm = flux_tile_bytes(BY) + slots * NPR * BY * FLUX_SLOT_W * sizeof(T);
   void (*kern)(StepArgs, CUtensorMap);
   // Where the blocks would take at most half of the SMs' slots (four 4-row
   // blocks each), each direction gets a layer of blocks of its own, and a
