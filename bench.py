@@ -847,24 +847,26 @@ def mixed_precision_leg(a, hb, stream, lim, flux, value_fp64, barrier, dist):
 # algorithmic bytes per active zone of one launch (FP64): every plane each
 # kernel must read or write once, 8 bytes a value
 KERNEL_BYTES = {
-    "k_flux": 8 * (8 + 2 * 21 + 2 * 8),       # prims once, FACE1+FACE2 geometry, F1+F2 out
-    "k_update": 8 * (8 + 8 + 21 + 40 + 2 + 2 * 8 + 1 + 8) + 4,  # pi, pb, CENT geo, conn, floors, 2 faces x2, emf, pf, pflag
+    # prims once, the 11 metric planes of the sparse form at FACE1 and FACE2, F1+F2 out
+    "k_flux": 8 * (8 + 2 * 11 + 2 * 8),
+    # pi, pb, the sparse form's CENT metric, conn, floors, 2 faces x2, emf, pf, pflag
+    "k_update": 8 * (8 + 8 + 14 + 40 + 2 + 2 * 8 + 1 + 8) + 4,
     "k_emf": 8 * (2 + 3 + 1),
-    "k_bsqflags": 8 * (8 + 21) + 1,
 }
 # with the per-zone HLL/LAXF switch the first substep's k_flux also reads the
-# CENT geometry (21 values) and writes the two flag bytes, the second reads
+# CENT geometry (14 values) and writes the two flag bytes, the second reads
 # the flux choice: averaged over the two launches of a step
-KERNEL_BYTES_SWITCH = {"k_flux": KERNEL_BYTES["k_flux"] + (8 * 21 + 2 + 1) / 2}
+KERNEL_BYTES_SWITCH = {"k_flux": KERNEL_BYTES["k_flux"] + (8 * 14 + 2 + 1) / 2}
 # FP64-pipe instructions (thread slots: adds, multiplies, comparisons and the
-# FMAs of division and square root) per active zone of one launch, from one
-# ncu capture of each kernel at 512^2 in the developed flow
+# FMAs of quotients and square roots) per active zone of one launch, from ncu
+# captures of both substeps' launches at 512^2 in the developed flow
 # (sm__inst_executed_pipe_fp64.sum x 32 / zones; profiles/k_flux_*, k_update_*;
-# the k_flux launch captured is a first substep, which also forms the flags)
-FP64_INSTR_PER_ZONE = {"k_flux": 3940, "k_update": 1983}
+# the first substep's k_flux also forms the flags: 2275 and 2065; k_update
+# 1320 and 1454)
+FP64_INSTR_PER_ZONE = {"k_flux": 2170, "k_update": 1387}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch from the same
-# captures, scaled by zone count
-TRAFFIC_512 = {"k_flux": 145.9e6, "k_update": 196.6e6}
+# captures (mean of both substeps), scaled by zone count
+TRAFFIC_512 = {"k_flux": 92.8e6, "k_update": 186.4e6}
 
 
 def main():
