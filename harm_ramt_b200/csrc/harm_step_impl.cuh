@@ -714,8 +714,9 @@ __global__ void __launch_bounds__(32 * BY, (BY == FLUX_BY_SMALL) ? 5 : 1)
   flux_block_dt(a, dt1, dt2, sh);
 }
 
-// FP64 faces.  FP64 issue and latency bound: 2080 FP64-pipe instructions a
-// zone (1900 with the sparse metric) at 128 registers (16 warps per SM).  What the layout is for:
+// FP64 faces.  FP64 issue and latency bound: 2255 FP64-pipe instructions a
+// zone (2065 with the sparse metric; 512^2 PARA, a launch that forms no
+// flags) at 128 registers (16 warps per SM).  What the layout is for:
 //  * all interface states are formed first, into shared memory (four slots a
 //    zone: the left and right state of its x1 and x2 face).  A warp takes one
 //    variable of the whole block and walks along the zones, so each slope and
