@@ -1044,9 +1044,14 @@ void launch_emf(int mixed, dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, co
 void launch_update(int mixed, int ffde, dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map,
                    const double* pi, const double* pb, double* pf, double c2)
 {
-  if (mixed) launch_update_mixed(ffde, g, b, s, a, map, pi, pb, pf, c2);
-  else if (ffde) update_launch<double, true>(g, b, s, a, map, pi, pb, pf, c2);
-  else update_launch<double, false>(g, b, s, a, map, pi, pb, pf, c2);
+  if (mixed) {
+    launch_update_mixed(ffde, g, b, s, a, map, pi, pb, pf, c2);
+  } else {
+    auto kern = ffde ? (a.sparse ? k_update<true, true> : k_update<true, false>)
+                     : (a.sparse ? k_update<false, true> : k_update<false, false>);
+    static bool attr[4] = {false, false, false, false};
+    update_launch(kern, attr[2 * (ffde != 0) + (a.sparse != 0)], g, b, s, a, map, pi, pb, pf, c2);
+  }
   if (!ffde) {
     if (a.pp.tryagain) k_update_tail_chain<<<148, 32 * TAIL_CHAIN, 0, s>>>(a, pi, pf);
     else k_update_tail<<<148, 64, 0, s>>>(a, pi, pf);

@@ -1217,53 +1217,54 @@ __device__ __forceinline__ void defer_zone(const StepArgs& a, long long z, int p
   a.worklist[atomicAdd(&a.sc->ndeferred, 1)] = (int)z;
 }
 
-// one zone's update by the general templates; returns its Newton iterations
-template <typename FT, bool FFDE>
-__device__ __noinline__ int update_general(const StepArgs& a, int i, int j, const double* pi, const double* pb,
-                                           double* pf, double c2, const double* sz, int plane_s)
+// The zone update by the general templates, in its parts: Ui = U(pi), with
+// pfz = pi; source_conn's terms; the RK combine of dUtoU (advance.c:273-286);
+// and the inversion, which returns its Newton iterations
+template <bool FFDE>
+__device__ __forceinline__ void conserved_general(const StepArgs& a, long long z, const Geo<double>& g,
+                                                  const double* pi, double* pfz, double* U)
 {
-  const long long pl = a.gr.plane, z = a.gr.at(i, j);
-  const double dt = a.sc->dt, gam = a.pp.gam;
-  Geo<double> g;
-  load_geo(a, CENT, z, g);
-  double U[NPR], pfz[NPR], dUr[NPR], dUg[NPR];
-  {
-    // Ui = U(pi)
-    double pr[NPR];
+  double pr[NPR];
 #pragma unroll
-    for (int k = 0; k < NPR; k++) pr[k] = __ldg(pi + k * pl + z);
+  for (int k = 0; k < NPR; k++) pr[k] = __ldg(pi + k * a.gr.plane + z);
 #pragma unroll
-    for (int k = 0; k < NPR; k++) pfz[k] = pr[k];
-    State<double> q;
-    state_of(pr, g, q);
-    flux_of<double, FFDE>(pr, q, 0, g, gam, U);
-    if (a.bsqf_fused) a.bsqf_fused[z] = bsq_flag(a, pr, q);  // get_bsqflags of the step's p
+  for (int k = 0; k < NPR; k++) pfz[k] = pr[k];
+  State<double> q;
+  state_of(pr, g, q);
+  flux_of<double, FFDE>(pr, q, 0, g, a.pp.gam, U);
+  if (a.bsqf_fused) a.bsqf_fused[z] = bsq_flag(a, pr, q);  // get_bsqflags of the step's p
+}
+template <bool FFDE>
+__device__ __forceinline__ void source_general(const StepArgs& a, long long z, const Geo<double>& g, const double* pb,
+                                               const double* sz, int plane_s, double* dUg)
+{
+  double pr[NPR];
+#pragma unroll
+  for (int k = 0; k < NPR; k++) pr[k] = __ldg(pb + k * a.gr.plane + z);
+  State<double> q;
+  state_of(pr, g, q);
+  double acc[4] = {0., 0., 0., 0.};
+#pragma unroll
+  for (int jj = 0; jj < 4; jj++) {
+    double row[4];
+    mhd_row<double, FFDE>(pr, jj, q, a.pp.gam, row);
+    source_row(row, jj, sz, plane_s, acc);
   }
-  flux_divergence<FT>(a, i, j, z, dUr);
-  {
-    double pr[NPR];
+  dUg[RHO] = 0. + g.g * 0.;
+  dUg[B1] = dUg[B2] = dUg[B3] = dUg[RHO];
 #pragma unroll
-    for (int k = 0; k < NPR; k++) pr[k] = __ldg(pb + k * pl + z);
-    State<double> q;
-    state_of(pr, g, q);
-    double acc[4] = {0., 0., 0., 0.};
+  for (int l = 0; l < 4; l++) dUg[UU + l] = 0. + g.g * acc[l];
+}
+__device__ __forceinline__ void combine_general(double cdt, const double* dUr, const double* dUg, double* U)
+{
 #pragma unroll
-    for (int jj = 0; jj < 4; jj++) {
-      double row[4];
-      mhd_row<double, FFDE>(pr, jj, q, gam, row);
-      source_row(row, jj, sz, plane_s, acc);
-    }
-    dUg[RHO] = 0. + g.g * 0.;
-    dUg[B1] = dUg[B2] = dUg[B3] = dUg[RHO];
-#pragma unroll
-    for (int l = 0; l < 4; l++) dUg[UU + l] = 0. + g.g * acc[l];
-  }
-  {
-    // the RK combine of dUtoU, advance.c:273-286
-    const double cdt = c2 * dt;
-#pragma unroll
-    for (int k = 0; k < NPR; k++) U[k] = 1.0 * U[k] + 0.0 * 0.0 + cdt * (dUr[k] + dUg[k]);
-  }
+  for (int k = 0; k < NPR; k++) U[k] = 1.0 * U[k] + 0.0 * 0.0 + cdt * (dUr[k] + dUg[k]);
+}
+template <bool FFDE>
+__device__ __forceinline__ int invert_general(const StepArgs& a, int i, int j, long long z, const Geo<double>& g,
+                                              const double* U, double* pfz, double* pf, const double* sz, int plane_s)
+{
+  const long long pl = a.gr.plane;
   if constexpr (FFDE) {
     // Utoprim_ffde, then fixup1zone's Lorentz-factor limit (the floors are
     // GRMHD-only, fixup.c:293); pflag is left as it was
@@ -1277,7 +1278,7 @@ __device__ __noinline__ int update_general(const StepArgs& a, int i, int j, cons
     int niter;
     // a deferred solve leaves its Newton state in the repair scratch (idle
     // until k_fixup_compute), NEWTON_STATE planes
-    const int pfl = utoprim_2d(U, g, pfz, gam, a.pp.gammafail, &niter, NEWTON_MAIN_CAP, a.fixbuf + z, pl);
+    const int pfl = utoprim_2d(U, g, pfz, a.pp.gam, a.pp.gammafail, &niter, NEWTON_MAIN_CAP, a.fixbuf + z, pl);
     if (pfl == NEWTON_DEFERRED || (a.pp.tryagain && pfl != 0)) {
       defer_zone(a, z, pfl, U);
       return 0;
@@ -1286,6 +1287,47 @@ __device__ __noinline__ int update_general(const StepArgs& a, int i, int j, cons
                 sz[(GEO_FLOOR + 1 - GEO_CONN) * plane_s]);
     return niter;
   }
+}
+
+// one zone's update by the general templates; returns its Newton iterations
+template <bool FFDE>
+__device__ __noinline__ int update_general(const StepArgs& a, int i, int j, const double* pi, const double* pb,
+                                           double* pf, double c2, const double* sz, int plane_s)
+{
+  const long long z = a.gr.at(i, j);
+  Geo<double> g;
+  load_geo(a, CENT, z, g);
+  double U[NPR], pfz[NPR], dUr[NPR], dUg[NPR];
+  conserved_general<FFDE>(a, z, g, pi, pfz, U);
+  flux_divergence<double>(a, i, j, z, dUr);
+  source_general<FFDE>(a, z, g, pb, sz, plane_s, dUg);
+  combine_general(c2 * a.sc->dt, dUr, dUg, U);
+  return invert_general<FFDE>(a, i, j, z, g, U, pfz, pf, sz, plane_s);
+}
+
+// block rows in launch order from both poles inward (0, last, 1, last-1,
+// ...): the zones near the axis take the most Newton iterations, and started
+// first their blocks no longer trail the kernel's last wave (developed 512^2
+// flow: 0.5256-0.5309 against 0.5333-0.5366 ms a step)
+__device__ __forceinline__ unsigned update_block_row()
+{
+  return (blockIdx.y & 1u) ? gridDim.y - 1u - (blockIdx.y >> 1) : (blockIdx.y >> 1);
+}
+// the block's connection and floor planes: issues the TMA copy (one thread)
+__device__ __forceinline__ void update_geo_load(double* sgeo, const CUtensorMap* map, unsigned by, uint64_t* bar)
+{
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
+    mbar_init(bar, 1);
+    mbar_expect_tx(bar, (uint32_t)upd_smem_bytes(blockDim.x, blockDim.y));
+    tma_load_3d(sgeo, map, (int)((blockIdx.x * blockDim.x + NG) & ~1u), (int)(by * blockDim.y + NG), GEO_CONN, bar);
+  }
+}
+// Newton iteration count (the reference's nstroke), one atomic per warp
+__device__ __forceinline__ void count_newton(const StepArgs& a, int niter)
+{
+  const unsigned mask = __activemask();
+  const unsigned it = __reduce_add_sync(mask, (unsigned)niter);
+  if ((int)(threadIdx.x & 31) == __ffs(mask) - 1) atomicAdd(&a.sc->newton_iters, (unsigned long long)it);
 }
 
 // advance_standard zone loop, advance.c:114-181, for one RK2 substep.
@@ -1299,7 +1341,7 @@ __device__ __noinline__ int update_general(const StepArgs& a, int i, int j, cons
 // us with the tail at 512^2).  A zone whose values leave the exact range goes
 // to update_general.  512^2 developed flow: 86 -> 50 us (first substep) and
 // 58 us (second), 3.9 TB/s; 1024^2 with the tail 300 -> 178 us.
-template <typename FT, bool FFDE, bool SP>
+template <bool FFDE, bool SP>
 __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepArgs a,
                                                    const __grid_constant__ CUtensorMap geo_map,
                                                    const double* __restrict__ pi, const double* __restrict__ pb,
@@ -1307,20 +1349,11 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
 {
   extern __shared__ __align__(128) double sgeo[];
   __shared__ uint64_t bar;
-  // block rows in launch order from both poles inward (0, last, 1, last-1,
-  // ...): the zones near the axis take the most Newton iterations, and
-  // started first their blocks no longer trail the kernel's last wave
-  // (developed 512^2 flow: 0.5256-0.5309 against 0.5333-0.5366 ms a step)
-  const unsigned by = (blockIdx.y & 1u) ? gridDim.y - 1u - (blockIdx.y >> 1) : (blockIdx.y >> 1);
+  const unsigned by = update_block_row();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = by * blockDim.y + threadIdx.y;
   const int W = upd_box_w(blockDim.x);
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    mbar_init(&bar, 1);
-    mbar_expect_tx(&bar, (uint32_t)upd_smem_bytes(blockDim.x, blockDim.y));
-    tma_load_3d(sgeo, &geo_map, (int)((blockIdx.x * blockDim.x + NG) & ~1u), (int)(by * blockDim.y + NG),
-                GEO_CONN, &bar);
-  }
+  update_geo_load(sgeo, &geo_map, by, &bar);
   const bool active = (i < a.gr.n1 && j < a.gr.n2);
   const long long pl = a.gr.plane, z = a.gr.at(active ? i : 0, active ? j : 0);
   const double dt = a.sc->dt, gam = a.pp.gam;
@@ -1333,7 +1366,7 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
   // the flux divergence first, while few registers are taken: its 28 loads
   // then start together (formed after U(pi), in small batches, they cost 20
   // of the kernel's 79 us at 512^2)
-  flux_divergence<FT>(a, active ? i : 0, active ? j : 0, z, dUr);
+  flux_divergence<double>(a, active ? i : 0, active ? j : 0, z, dUr);
   {
     const double* base = a.geo + (long long)CENT * GEO_PER_LOC * pl + z;
 #pragma unroll
@@ -1394,7 +1427,7 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
   if constexpr (FFDE) {
     utoprim_ffde_x<SP>(ex, U, c, gn, sg, pfz, a.pp.gammamax);
     if (!ex.ok()) {
-      update_general<FT, FFDE>(a, i, j, pi, pb, pf, c2, sz, plane_s);
+      update_general<FFDE>(a, i, j, pi, pb, pf, c2, sz, plane_s);
       return;
     }
 #pragma unroll
@@ -1406,7 +1439,7 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
     const int pfl = utoprim_2d_x<SP>(ex, U, c, gn, sg, pfz, gam, a.pp.gammafail, &niter, NEWTON_MAIN_CAP, a.fixbuf + z, pl,
                                  false);
     if (!ex.ok()) {
-      niter = update_general<FT, FFDE>(a, i, j, pi, pb, pf, c2, sz, plane_s);
+      niter = update_general<FFDE>(a, i, j, pi, pb, pf, c2, sz, plane_s);
     } else {
       if (a.bsqf_fused) a.bsqf_fused[z] = bf;
       if (pfl == NEWTON_DEFERRED || (a.pp.tryagain && pfl != 0)) {
@@ -1420,21 +1453,17 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
                     sz[(GEO_FLOOR + 1 - GEO_CONN) * plane_s]);
       }
     }
-    // Newton iteration count (the reference's nstroke), one atomic per warp
-    const unsigned mask = __activemask();
-    const unsigned it = __reduce_add_sync(mask, (unsigned)niter);
-    if ((int)(threadIdx.x & 31) == __ffs(mask) - 1) atomicAdd(&a.sc->newton_iters, (unsigned long long)it);
+    count_newton(a, niter);
   }
 }
 
 // launches a k_update instance (its dynamic shared memory limit raised once
 // to the largest box of the tile shapes harm_set_tiles accepts: 42 planes x
 // at most 128 threads)
-template <typename FT, bool FFDE, bool SP>
-inline void update_launch_sp(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map, const double* pi,
-                             const double* pb, double* pf, double c2)
+inline void update_launch(void (*kern)(StepArgs, CUtensorMap, const double*, const double*, double*, double), bool& attr,
+                          dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map, const double* pi,
+                          const double* pb, double* pf, double c2)
 {
-  static bool attr = false;
   if (!attr) {
     size_t mx = 0;
     for (int by = 1; by <= 128; by++) {
@@ -1442,17 +1471,10 @@ inline void update_launch_sp(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, 
       const size_t v = upd_smem_bytes(bx + (bx & 1), by);
       if (v > mx) mx = v;
     }
-    cudaFuncSetAttribute(k_update<FT, FFDE, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx);
     attr = true;
   }
-  k_update<FT, FFDE, SP><<<g, b, upd_smem_bytes(b.x, b.y), s>>>(a, map, pi, pb, pf, c2);
-}
-template <typename FT, bool FFDE>
-inline void update_launch(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map, const double* pi,
-                          const double* pb, double* pf, double c2)
-{
-  if (a.sparse) update_launch_sp<FT, FFDE, true>(g, b, s, a, map, pi, pb, pf, c2);
-  else update_launch_sp<FT, FFDE, false>(g, b, s, a, map, pi, pb, pf, c2);
+  kern<<<g, b, upd_smem_bytes(b.x, b.y), s>>>(a, map, pi, pb, pf, c2);
 }
 
 // ---------------------------------------------------------------- end of step
