@@ -164,9 +164,10 @@ struct Exact {
 // The same with numerators down to the smallest subnormal number, for groups
 // that carry such numbers (the field ahead of the front it spreads with): the
 // quotient is formed 2^400 times as large and scaled down.  Scaling rounds a
-// second time where the quotient is subnormal: there the residual of the
-// rounded value, exact at the larger scale, tells whether it is off by more
-// than half the spacing 2^-1074, and moves it by one.
+// second time where the quotient is subnormal (one just below 2^-1022 may
+// become that number): there the residual of the rounded value, exact at the
+// larger scale, tells whether it is off by more than half the spacing 2^-1074,
+// and moves it by one.
 struct ExactTiny : Exact {
   HD_INLINE double div(double a, const Recip& d)
   {
@@ -174,7 +175,7 @@ struct ExactTiny : Exact {
     numerator(as);
     const double q = quot(as, d) * 0x1p-400;
     const double r = fma(-d.b, q * 0x1p400, as);
-    const bool off = fabs(q) < 0x1p-1022 && fabs(r) > fabs(d.b) * 0x1p-675;
+    const bool off = fabs(q) <= 0x1p-1022 && fabs(r) > fabs(d.b) * 0x1p-675;
     const bool up = (r > 0.) == (as > 0.);
     const uint64_t u = bits_of(q) + (off ? (up ? 1 : ~0ull) : 0);
 #ifdef __CUDA_ARCH__

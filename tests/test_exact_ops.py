@@ -60,3 +60,17 @@ def test_out_of_range_is_reported(where, nudge):
     assert not ec.evaluate(where, False, np.ones(len(wild)), wild, nudge)[1].any()
     wild = np.array([0.0, -0.0, -1.0, 5e-324, 2.0 ** -201, 2.0 ** 61, np.inf, np.nan])
     assert not ec.evaluate(where, True, wild, wild, nudge)[1].any()
+
+
+@pytest.mark.parametrize("where,nudge", PLACES)
+def test_quotients_next_to_the_smallest_normal(where, nudge):
+    """a / b half a spacing or less below 2^-1022 and a few spacings around it."""
+    b = np.concatenate([1.0 + np.arange(1, 256) / 256.0, 1.0 + 2.0 ** -52 * np.arange(1, 64), 2.0 - 2.0 ** -52 * np.arange(1, 64)])
+    b, k = (x.ravel() for x in np.meshgrid(b, np.arange(-8, 17), indexing="ij"))
+    for sign in (1.0, -1.0):
+        for s in (-1, 0, 3):
+            a, d = sign * (b * 2.0 ** -1022 - k * 2.0 ** -1074), np.ldexp(b, s)
+            a = np.ldexp(a, s) if s > 0 else a
+            q, ok = ec.evaluate(where, 2, a, d, nudge)
+            assert ok.all()
+            assert np.array_equal(q, a / d)
