@@ -227,10 +227,10 @@ __device__ __forceinline__ void state_x(EX& ex, const double* pr, const double* 
   const double gamma = ex.sqrt_of(1. + qsq_x<SP>(pr, c));
   ex.need(gamma <= limit);
   q.gamma = gamma;
-  q.ucon[0] = Exact::quot(gamma, l.alpha);
+  q.ucon[0] = EX::quot(gamma, l.alpha);
 #pragma unroll
   for (int k = 0; k < 3; k++)
-    q.ucon[1 + k] = (SP && k > 0) ? pr[U1 + k] : pr[U1 + k] - Exact::quot(gamma * l.beta[k], l.alpha);
+    q.ucon[1 + k] = (SP && k > 0) ? pr[U1 + k] : pr[U1 + k] - EX::quot(gamma * l.beta[k], l.alpha);
   lower_cov<SP>(q.ucon, c, q.ucov);
   q.bcon[0] = pr[B1] * q.ucov[1] + pr[B2] * q.ucov[2] + pr[B3] * q.ucov[3];
   q.ut = ex.rcp(q.ucon[0]);
@@ -953,7 +953,7 @@ __device__ __forceinline__ double utsq_calc_x(ExactTiny& ex, const U2PCtx& c, do
 {
   const double Wsq = W * W, W4 = Wsq * Wsq;
   const double den = W4 + 2. * c.Bsq * Wsq * W + Wsq * (c.Bsq * c.Bsq - c.Qtsq) - c.QdotBsq * (2. * W + c.Bsq);
-  return ex.Exact::div(c.Bsq * c.QdotBsq + W * (2. * c.QdotBsq + c.Qtsq * W), ex.rcp(den));
+  return ex.div_normal(c.Bsq * c.QdotBsq + W * (2. * c.QdotBsq + c.Qtsq * W), ex.rcp(den));
 }
 
 __device__ __forceinline__ int newton_vsq_x(ExactTiny& ex, const U2PCtx& c, double& x0, double& x1, double gammafail,
@@ -980,19 +980,19 @@ __device__ __forceinline__ int newton_vsq_x(ExactTiny& ex, const U2PCtx& c, doub
     const double W = x0, vsq = x1, Wsq = W * W, W3 = Wsq * W, gtmp = 1. - vsq;
     const double sq = ex.sqrt_of(gtmp);
     const Recip r2 = ex.rcp_from(Wsq, rW.y * rW.y), r3 = ex.rcp_from(W3, r2.y * rW.y);
-    const double p_tmp = Exact::quot((gam - 1.) * (W * gtmp - c.D * sq), rgam);
-    const double dPdW = Exact::quot((gam - 1.) * gtmp, rgam);
-    const double dPdvsq = Exact::quot((gam - 1.) * (Exact::quot(0.5 * c.D, ex.rcp(sq)) - W), rgam);
+    const double p_tmp = ExactTiny::quot((gam - 1.) * (W * gtmp - c.D * sq), rgam);
+    const double dPdW = ExactTiny::quot((gam - 1.) * gtmp, rgam);
+    const double dPdvsq = ExactTiny::quot((gam - 1.) * (ExactTiny::quot(0.5 * c.D, ex.rcp(sq)) - W), rgam);
     const double BW = Bsq + W;
-    const double t2 = c.Qtsq - vsq * (BW * BW) + Exact::quot(QdotBsq * (Bsq + 2 * W), r2);
-    const double t3 = c.Qdotn - (Bsq * (1 + vsq)) / 2. + 0.5 * Exact::quot(QdotBsq, r2) - W + p_tmp;
-    const double QW3 = Exact::quot(QdotBsq, r3), s = -1 + dPdW - QW3;
+    const double t2 = c.Qtsq - vsq * (BW * BW) + ExactTiny::quot(QdotBsq * (Bsq + 2 * W), r2);
+    const double t3 = c.Qdotn - (Bsq * (1 + vsq)) / 2. + 0.5 * ExactTiny::quot(QdotBsq, r2) - W + p_tmp;
+    const double QW3 = ExactTiny::quot(QdotBsq, r3), s = -1 + dPdW - QW3;
     double dx0 = (-Bsq / 2. + dPdvsq) * t2 + (BW * BW) * t3;
     double dx1 = -(s * t2) - 2 * (vsq + QW3) * BW * t3;
-    const double detJ = BW * (s * BW + Exact::quot((Bsq - 2 * dPdvsq) * (QdotBsq + vsq * W3), r3));
+    const double detJ = BW * (s * BW + ExactTiny::quot((Bsq - 2 * dPdvsq) * (QdotBsq + vsq * W3), r3));
     const Recip rd = ex.rcp(fabs(detJ));
-    dx0 = Exact::quot((detJ < 0.) ? dx0 : -dx0, rd);
-    dx1 = Exact::quot((detJ < 0.) ? dx1 : -dx1, rd);
+    dx0 = ExactTiny::quot((detJ < 0.) ? dx0 : -dx0, rd);
+    dx1 = ExactTiny::quot((detJ < 0.) ? dx1 : -dx1, rd);
     if (((n_iter + 1) % 10) == 0) {
       const double r = cycle_break_uniform(x0, x1, n_iter);
       dx0 *= r;
@@ -1004,8 +1004,8 @@ __device__ __forceinline__ int newton_vsq_x(ExactTiny& ex, const U2PCtx& c, doub
     rW = ex.rcp(x0);
     x1 += dx1;
     // where x1 is zero the reference takes |dx1| itself
-    errx = (Exact::quot(fabs(dx0), rW) + Exact::quot(fabs(dx1), ex.rcp((x1 == 0.) ? 1. : fabs(x1)))) / 2.;
-    ex.need(!(Exact::quot(x0, rwg) > W_TOO_BIG));
+    errx = (ExactTiny::quot(fabs(dx0), rW) + ExactTiny::quot(fabs(dx1), ex.rcp((x1 == 0.) ? 1. : fabs(x1)))) / 2.;
+    ex.need(!(ExactTiny::quot(x0, rwg) > W_TOO_BIG));
     x1 = (x1 < 0.) ? 0.0 : x1;
     x1 = (x1 > 1.) ? vsq_too_big : x1;
     if (((errx_old == errx) || (errx_oldest == errx)) && (errx < MIN_NEWT_TOL)) errx = -errx;
@@ -1036,12 +1036,12 @@ __device__ __forceinline__ int utoprim_2d_x(ExactTiny& ex, const double* U, cons
   double Ut[NPR];
   const Recip rs = ex.rcp(sg);
   const double ngn = -gn[0];
-  const Recip ral = ex.rcp(Exact::quot(1., ex.rcp(ex.sqrt_of(ngn))));  // alpha
+  const Recip ral = ex.rcp(ExactTiny::quot(1., ex.rcp(ex.sqrt_of(ngn))));  // alpha
   const double alpha = ral.b;
   {
     double Ug[NPR];
 #pragma unroll
-    for (int k = 0; k < B1; k++) Ug[k] = ex.Exact::div(U[k], rs);
+    for (int k = 0; k < B1; k++) Ug[k] = ex.div_normal(U[k], rs);
 #pragma unroll
     for (int k = B1; k <= B3; k++) Ug[k] = ex.div(U[k], rs);
     Ug[UU] += -Ug[RHO];
@@ -1062,7 +1062,7 @@ __device__ __forceinline__ int utoprim_2d_x(ExactTiny& ex, const double* U, cons
   raise_con<SP>(Q, gn, Qcon);
   const double QdotB = Q[1] * B[0] + Q[2] * B[1] + Q[3] * B[2];
   x.QdotBsq = QdotB * QdotB;
-  const double nlapse = -ex.sqrt_of(Exact::quot(1., ex.rcp(ngn)));
+  const double nlapse = -ex.sqrt_of(ExactTiny::quot(1., ex.rcp(ngn)));
   x.Qdotn = Qcon[0] * nlapse;
   x.Qtsq = Q[0] * Qcon[0] + Q[1] * Qcon[1] + Q[2] * Qcon[2] + Q[3] * Qcon[3] + x.Qdotn * x.Qdotn;
   x.D = Ut[RHO];
@@ -1081,7 +1081,7 @@ __device__ __forceinline__ int utoprim_2d_x(ExactTiny& ex, const double* U, cons
   x.wglobal = w0;
   double W = w0 * (1. + utsq);
   double x0 = fabs(W), ut = fabs(utsq_calc_x(ex, x, W));
-  double x1 = ex.Exact::div(ut, ex.rcp(ut + 1.));
+  double x1 = ex.div_normal(ut, ex.rcp(ut + 1.));
   const int ret = newton_vsq_x(ex, x, x0, x1, gammafail, *niter, maxit, nst, nss, resume);
   if (ret == NEWTON_DEFERRED) return NEWTON_DEFERRED;
 #pragma unroll
@@ -1089,14 +1089,14 @@ __device__ __forceinline__ int utoprim_2d_x(ExactTiny& ex, const double* U, cons
   if (ret != 0) return ret * 100 + 1;
   W = x0;
   if (W == FAIL_VAL) return 1;
-  if (Exact::quot(W, ex.rcp(w0)) > W_TOO_BIG) return PF_CONVW;
+  if (ExactTiny::quot(W, ex.rcp(w0)) > W_TOO_BIG) return PF_CONVW;
   utsq = utsq_calc_x(ex, x, W);
   if ((utsq < 0.) && (fabs(utsq) < 1.0e-13)) utsq = fabs(utsq);
   if (utsq < 0. || utsq > utsq_too_big) return PF_CONVUTSQ2;
   const double gamma = ex.sqrt_of(1. + utsq);
-  const double rho0 = ex.Exact::div(x.D, ex.rcp(gamma));
-  const double w = Exact::quot(W, ex.rcp(gamma * gamma));
-  const double p = ex.Exact::div((gam - 1.) * (w - rho0), ex.rcp(gam));
+  const double rho0 = ex.div_normal(x.D, ex.rcp(gamma));
+  const double w = ExactTiny::quot(W, ex.rcp(gamma * gamma));
+  const double p = ex.div_normal((gam - 1.) * (w - rho0), ex.rcp(gam));
   const double u = w - (rho0 + p);
   int pfl = 0;
   if ((rho0 <= 0.) || (u <= 0.)) {
@@ -1111,10 +1111,10 @@ __device__ __forceinline__ int utoprim_2d_x(ExactTiny& ex, const double* U, cons
 #pragma unroll
   for (int i = 1; i < 4; i++) {
     const double Qt = (SP && i > 1) ? Qcon[i] : Qcon[i] + (gn[i] * nlapse) * x.Qdotn;
-    const double t1 = ex.Exact::div(-gamma * Qt, r1), n2 = gamma * QdotB * B[i - 1];
+    const double t1 = ex.div_normal(-gamma * Qt, r1), n2 = gamma * QdotB * B[i - 1];
     // the field's part is watched only where the other does not drown it
     ex.numerator((fabs(t1) > 1.e-150) ? 0. : n2);
-    pr[U1 + i - 1] = t1 - Exact::quot(n2, r2);
+    pr[U1 + i - 1] = t1 - ExactTiny::quot(n2, r2);
   }
   return pfl;
 }
@@ -1131,18 +1131,18 @@ __device__ __forceinline__ void utoprim_ffde_x(ExactTiny& ex, const double* U, c
     S[k] = ex.div(U[U1 + k], rs);
     B[k] = ex.div(U[B1 + k], rs);
   }
-  const double alphasq = Exact::quot(1., ex.rcp(-gn[0]));
+  const double alphasq = ExactTiny::quot(1., ex.rcp(-gn[0]));
   double bv[3];
   lower_space<SP>(B, c, bv);
   const double b1 = bv[0], b2 = bv[1], b3 = bv[2];
   const double Bsq = b1 * B[0] + b2 * B[1] + b3 * B[2];
-  const double o = Exact::quot(1., ex.rcp(Bsq * sg));
+  const double o = ExactTiny::quot(1., ex.rcp(Bsq * sg));
   const double E[3] = {(b2 * S[2] - b3 * S[1]) * o, (b3 * S[0] - b1 * S[2]) * o, (b1 * S[1] - b2 * S[0]) * o};
   double ev[3];
   lower_space<SP>(E, c, ev);
   const double e1 = ev[0], e2 = ev[1], e3 = ev[2];
   const double Esq = E[0] * e1 + E[1] * e2 + E[2] * e3;
-  const double gammasq = ex.Exact::div(Bsq, ex.rcp(Bsq - Esq));
+  const double gammasq = ex.div_normal(Bsq, ex.rcp(Bsq - Esq));
   ex.need(gammasq <= gammamax * gammamax && gammasq >= 1.0);
   double v[4], uc[4];
   v[1] = alphasq * (-gn[1] + (e2 * b3 - e3 * b2) * o);
@@ -1152,7 +1152,7 @@ __device__ __forceinline__ void utoprim_ffde_x(ExactTiny& ex, const double* U, c
                        : c[1] * v[1] + c[2] * v[2] + c[3] * v[3] + c[5] * v[1] * v[2] + c[6] * v[1] * v[3] +
                              c[8] * v[2] * v[3];
   const double discr = +c[0] + c[4] * v[1] * v[1] + c[7] * v[2] * v[2] + c[9] * v[3] * v[3] + 2. * d2;
-  uc[0] = Exact::quot(1., ex.rcp(ex.sqrt_of(-discr)));
+  uc[0] = ExactTiny::quot(1., ex.rcp(ex.sqrt_of(-discr)));
 #pragma unroll
   for (int j = 1; j < 4; j++) pr[U1 - 1 + j] = v[j] * uc[0];
 #pragma unroll
@@ -1421,7 +1421,7 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
 #pragma unroll
     for (int k = 0; k < NPR; k++) {
       const double d = (k >= UU && k <= U3) ? dUr[k] + sg * acc[k - UU] : dUr[k];
-      U[k] = U[k] + cdt * d;
+      U[k] = (U[k] + 0.) + cdt * d;  // (+ 0., as dUtoU has it: no zero stays negative)
     }
   }
   if constexpr (FFDE) {

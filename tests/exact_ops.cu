@@ -1,6 +1,7 @@
 // The quotients and roots of harm_exact.cuh over arrays, on the host (with a
 // shifted seed) and on the device.  root: 0 a / b, 1 sqrt(a), 2 a / b down to
-// subnormal numbers.
+// subnormal numbers, 3 the same for normal ones, 4 and 5 a / (b b) and
+// a / ((b b) b) with reciprocals from that of b.
 #include <cuda_runtime.h>
 
 #include "../harm_ramt_b200/csrc/harm_exact.cuh"
@@ -12,6 +13,11 @@ HD_INLINE void one(int root, double a, double b, int nudge, double* q, unsigned 
   if (root == 2) {
     ExactTiny ex;
     *q = ex.div(a, ex.rcp(b, nudge));
+    *ok = ex.ok();
+  } else if (root > 2) {
+    ExactTiny ex;
+    const Recip r1 = ex.rcp(b, nudge), r2 = ex.rcp_from(b * b, r1.y * r1.y), r3 = ex.rcp_from((b * b) * b, r2.y * r1.y);
+    *q = ex.div_normal(a, root == 3 ? r1 : (root == 4 ? r2 : r3));
     *ok = ex.ok();
   } else {
     Exact ex;

@@ -62,6 +62,27 @@ def test_out_of_range_is_reported(where, nudge):
     assert not ec.evaluate(where, True, wild, wild, nudge)[1].any()
 
 
+def _same_bits(q, ref):
+    return np.array_equal(q.view(np.uint64), ref.view(np.uint64))
+
+
+@pytest.mark.parametrize("where,nudge", PLACES)
+@pytest.mark.parametrize("root", [2, 3])
+def test_signs_of_zero(where, nudge, root):
+    """A quotient of zero, and one that rounds to zero, keeps its sign (in the
+    form that the primitives are made with)."""
+    r = np.random.default_rng(10)
+    b = np.concatenate([r.uniform(1, 2, 500) * 2.0 ** r.integers(-60, 19, 500), 1.0 + np.arange(64) / 64.0])
+    a = np.concatenate([np.zeros_like(b), -np.zeros_like(b)])
+    b = np.tile(b, 2)
+    q, ok = ec.evaluate(where, root, a, b, nudge)
+    assert ok.all() and _same_bits(q, a / b)
+    if root == 2:
+        a, b = np.where(np.signbit(a), -5e-324, 5e-324), np.abs(b) + 2.5
+        q, ok = ec.evaluate(where, root, a, np.minimum(b, 2.0 ** 59), nudge)
+        assert ok.all() and _same_bits(q, a / np.minimum(b, 2.0 ** 59))
+
+
 @pytest.mark.parametrize("where,nudge", PLACES)
 def test_quotients_next_to_the_smallest_normal(where, nudge):
     """a / b half a spacing or less below 2^-1022 and a few spacings around it."""
