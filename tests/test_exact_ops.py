@@ -95,3 +95,23 @@ def test_quotients_next_to_the_smallest_normal(where, nudge):
             q, ok = ec.evaluate(where, 2, a, d, nudge)
             assert ok.all()
             assert np.array_equal(q, a / d)
+
+
+@pytest.mark.parametrize("where,nudge", PLACES)
+@pytest.mark.parametrize("root,power", [(4, 2), (5, 3)])
+def test_quotients_by_powers(where, nudge, root, power):
+    """Quotients by W^2 and W^3 whose reciprocals come from 1 / W, as in the
+    Newton step: over random W, W next to powers of two and thirds, and
+    numerators that put the quotient next to a tie."""
+    r = np.random.default_rng(11)
+    n = 1 << 18
+    e = 2.0 ** -52 * np.arange(1, 4096)
+    W = np.concatenate([r.uniform(1, 2, n) * 2.0 ** r.integers(-60, 19, n), 1.0 + e, 2.0 - e, 4.0 / 3.0 + e, 1.5 - e,
+                        np.sqrt(2.0) + e, np.cbrt(2.0) - e])
+    d = W * W if power == 2 else (W * W) * W
+    a, b = ec.hard_quotients(200)
+    near = (r.integers(1 << 52, 1 << 53, len(W)) + 0.5) * 2.0 ** -52 * d
+    for num in (r.uniform(-1, 1, len(W)), near, d, np.nextafter(d, 0.0), -np.nextafter(d, np.inf), r.choice(a, len(W))):
+        q, ok = ec.evaluate(where, root, num, W, nudge)
+        assert ok.all()
+        assert np.array_equal(q, num / d)
