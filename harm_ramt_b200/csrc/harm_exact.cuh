@@ -113,6 +113,8 @@ struct Exact {
     return (h - lo > m) ? h - lo : m;
 #endif
   }
+  // a factor of sums and products that are to stay finite: |a| below 2^528
+  HD_INLINE void bounded(double a) { num = above(num, hi_word(a) & 0x7fffffffu, 0); }
   // a value that only the general code handles
   HD_INLINE void need(bool c) { pos = c ? pos : 0xffffffffu; }
   // a numerator: zero (a quotient of zero is exact), or in the range (its

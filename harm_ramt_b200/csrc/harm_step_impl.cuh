@@ -313,6 +313,10 @@ __device__ __forceinline__ void side_x(EX& ex, const double* pr, const StateX& q
     x.U[XB] = Bo * sg;
     x.U[XB3] = pr[B3] * sg;
   }
+  // (a density or internal energy without bound can leave the wavespeeds in
+  // range -- where the sum below is not positive -- and the fluxes infinite)
+  ex.bounded(pr[RHO]);
+  if (!FFDE) ex.bounded(pr[UU]);
   // vchar and simplefast
   const double WW0 = pr[RHO] + gam * pr[UU];
   const bool wpos = WW0 > 0.;
@@ -394,8 +398,8 @@ __device__ __forceinline__ void face_flux_x(EX& ex, const StepArgs& a, const Fac
   cmax = fabs(rmax(0., cmax));
   const double ctop = rmax(cmax, cmin), cc = cmax * cmin;
   const Recip sum = ex.rcp(cmax + cmin);
-  // an in-range divisor keeps both forms finite, so the form that
-  // choose_flux weighs with 0 adds nothing
+  // an in-range divisor and bounded states keep both forms finite, so the form
+  // that choose_flux weighs with 0 adds nothing
 #pragma unroll
   for (int k = 0; k < NX; k++) {
     const double dU = sr.U[k] - sl.U[k];
