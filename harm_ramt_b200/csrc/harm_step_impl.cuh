@@ -315,8 +315,7 @@ __device__ __forceinline__ void side_x(EX& ex, const double* pr, const StateX& q
   }
   // (a density or internal energy without bound can leave the wavespeeds in
   // range -- where the sum below is not positive -- and the fluxes infinite)
-  ex.bounded(pr[RHO]);
-  if (!FFDE) ex.bounded(pr[UU]);
+  ex.bounded(FFDE ? pr[RHO] : (gam - 1.) * pr[UU] + pr[RHO] + pr[UU]);
   // vchar and simplefast
   const double WW0 = pr[RHO] + gam * pr[UU];
   const bool wpos = WW0 > 0.;
@@ -1221,54 +1220,54 @@ __device__ __forceinline__ void defer_zone(const StepArgs& a, long long z, int p
   a.worklist[atomicAdd(&a.sc->ndeferred, 1)] = (int)z;
 }
 
-// The zone update by the general templates, in its parts: Ui = U(pi), with
-// pfz = pi; source_conn's terms; the RK combine of dUtoU (advance.c:273-286);
-// and the inversion, which returns its Newton iterations
+// one zone's update by the general templates; returns its Newton iterations
+// (the mixed form's update is this one too, in k_update_mixed's own text)
 template <bool FFDE>
-__device__ __forceinline__ void conserved_general(const StepArgs& a, long long z, const Geo<double>& g,
-                                                  const double* pi, double* pfz, double* U)
+__device__ __noinline__ int update_general(const StepArgs& a, int i, int j, const double* pi, const double* pb,
+                                           double* pf, double c2, const double* sz, int plane_s)
 {
-  double pr[NPR];
+  const long long pl = a.gr.plane, z = a.gr.at(i, j);
+  const double dt = a.sc->dt, gam = a.pp.gam;
+  Geo<double> g;
+  load_geo(a, CENT, z, g);
+  double U[NPR], pfz[NPR], dUr[NPR], dUg[NPR];
+  {
+    // Ui = U(pi)
+    double pr[NPR];
 #pragma unroll
-  for (int k = 0; k < NPR; k++) pr[k] = __ldg(pi + k * a.gr.plane + z);
+    for (int k = 0; k < NPR; k++) pr[k] = __ldg(pi + k * pl + z);
 #pragma unroll
-  for (int k = 0; k < NPR; k++) pfz[k] = pr[k];
-  State<double> q;
-  state_of(pr, g, q);
-  flux_of<double, FFDE>(pr, q, 0, g, a.pp.gam, U);
-  if (a.bsqf_fused) a.bsqf_fused[z] = bsq_flag(a, pr, q);  // get_bsqflags of the step's p
-}
-template <bool FFDE>
-__device__ __forceinline__ void source_general(const StepArgs& a, long long z, const Geo<double>& g, const double* pb,
-                                               const double* sz, int plane_s, double* dUg)
-{
-  double pr[NPR];
-#pragma unroll
-  for (int k = 0; k < NPR; k++) pr[k] = __ldg(pb + k * a.gr.plane + z);
-  State<double> q;
-  state_of(pr, g, q);
-  double acc[4] = {0., 0., 0., 0.};
-#pragma unroll
-  for (int jj = 0; jj < 4; jj++) {
-    double row[4];
-    mhd_row<double, FFDE>(pr, jj, q, a.pp.gam, row);
-    source_row(row, jj, sz, plane_s, acc);
+    for (int k = 0; k < NPR; k++) pfz[k] = pr[k];
+    State<double> q;
+    state_of(pr, g, q);
+    flux_of<double, FFDE>(pr, q, 0, g, gam, U);
+    if (a.bsqf_fused) a.bsqf_fused[z] = bsq_flag(a, pr, q);  // get_bsqflags of the step's p
   }
-  dUg[RHO] = 0. + g.g * 0.;
-  dUg[B1] = dUg[B2] = dUg[B3] = dUg[RHO];
+  flux_divergence<double>(a, i, j, z, dUr);
+  {
+    double pr[NPR];
 #pragma unroll
-  for (int l = 0; l < 4; l++) dUg[UU + l] = 0. + g.g * acc[l];
-}
-__device__ __forceinline__ void combine_general(double cdt, const double* dUr, const double* dUg, double* U)
-{
+    for (int k = 0; k < NPR; k++) pr[k] = __ldg(pb + k * pl + z);
+    State<double> q;
+    state_of(pr, g, q);
+    double acc[4] = {0., 0., 0., 0.};
 #pragma unroll
-  for (int k = 0; k < NPR; k++) U[k] = 1.0 * U[k] + 0.0 * 0.0 + cdt * (dUr[k] + dUg[k]);
-}
-template <bool FFDE>
-__device__ __forceinline__ int invert_general(const StepArgs& a, int i, int j, long long z, const Geo<double>& g,
-                                              const double* U, double* pfz, double* pf, const double* sz, int plane_s)
-{
-  const long long pl = a.gr.plane;
+    for (int jj = 0; jj < 4; jj++) {
+      double row[4];
+      mhd_row<double, FFDE>(pr, jj, q, gam, row);
+      source_row(row, jj, sz, plane_s, acc);
+    }
+    dUg[RHO] = 0. + g.g * 0.;
+    dUg[B1] = dUg[B2] = dUg[B3] = dUg[RHO];
+#pragma unroll
+    for (int l = 0; l < 4; l++) dUg[UU + l] = 0. + g.g * acc[l];
+  }
+  {
+    // the RK combine of dUtoU, advance.c:273-286
+    const double cdt = c2 * dt;
+#pragma unroll
+    for (int k = 0; k < NPR; k++) U[k] = 1.0 * U[k] + 0.0 * 0.0 + cdt * (dUr[k] + dUg[k]);
+  }
   if constexpr (FFDE) {
     // Utoprim_ffde, then fixup1zone's Lorentz-factor limit (the floors are
     // GRMHD-only, fixup.c:293); pflag is left as it was
@@ -1282,7 +1281,7 @@ __device__ __forceinline__ int invert_general(const StepArgs& a, int i, int j, l
     int niter;
     // a deferred solve leaves its Newton state in the repair scratch (idle
     // until k_fixup_compute), NEWTON_STATE planes
-    const int pfl = utoprim_2d(U, g, pfz, a.pp.gam, a.pp.gammafail, &niter, NEWTON_MAIN_CAP, a.fixbuf + z, pl);
+    const int pfl = utoprim_2d(U, g, pfz, gam, a.pp.gammafail, &niter, NEWTON_MAIN_CAP, a.fixbuf + z, pl);
     if (pfl == NEWTON_DEFERRED || (a.pp.tryagain && pfl != 0)) {
       defer_zone(a, z, pfl, U);
       return 0;
@@ -1291,22 +1290,6 @@ __device__ __forceinline__ int invert_general(const StepArgs& a, int i, int j, l
                 sz[(GEO_FLOOR + 1 - GEO_CONN) * plane_s]);
     return niter;
   }
-}
-
-// one zone's update by the general templates; returns its Newton iterations
-template <bool FFDE>
-__device__ __noinline__ int update_general(const StepArgs& a, int i, int j, const double* pi, const double* pb,
-                                           double* pf, double c2, const double* sz, int plane_s)
-{
-  const long long z = a.gr.at(i, j);
-  Geo<double> g;
-  load_geo(a, CENT, z, g);
-  double U[NPR], pfz[NPR], dUr[NPR], dUg[NPR];
-  conserved_general<FFDE>(a, z, g, pi, pfz, U);
-  flux_divergence<double>(a, i, j, z, dUr);
-  source_general<FFDE>(a, z, g, pb, sz, plane_s, dUg);
-  combine_general(c2 * a.sc->dt, dUr, dUg, U);
-  return invert_general<FFDE>(a, i, j, z, g, U, pfz, pf, sz, plane_s);
 }
 
 // block rows in launch order from both poles inward (0, last, 1, last-1,

@@ -59,7 +59,18 @@ __global__ void __launch_bounds__(128, 4) k_update_mixed(StepArgs a, const __gri
   double U[NPR], pfz[NPR], dUr[NPR], dUg[NPR];
   if (active) {
     load_geo(a, CENT, z, g);
-    conserved_general<FFDE>(a, z, g, pi, pfz, U);
+    {
+      // Ui = U(pi)
+      double pr[NPR];
+#pragma unroll
+      for (int k = 0; k < NPR; k++) pr[k] = __ldg(pi + k * pl + z);
+#pragma unroll
+      for (int k = 0; k < NPR; k++) pfz[k] = pr[k];
+      State<double> q;
+      state_of(pr, g, q);
+      flux_of<double, FFDE>(pr, q, 0, g, gam, U);
+      if (a.bsqf_fused) a.bsqf_fused[z] = bsq_flag(a, pr, q);  // get_bsqflags of the step's p
+    }
     flux_divergence<float>(a, i, j, z, dUr);
   }
   if (!mbar_wait(&bar, 0)) {
@@ -69,10 +80,50 @@ __global__ void __launch_bounds__(128, 4) k_update_mixed(StepArgs a, const __gri
   if (!active) return;
   const int plane_s = blockDim.y * W;
   const double* sz = sgeo + threadIdx.y * W + threadIdx.x + 1;
-  source_general<FFDE>(a, z, g, pb, sz, plane_s, dUg);
-  combine_general(c2 * dt, dUr, dUg, U);
-  const int niter = invert_general<FFDE>(a, i, j, z, g, U, pfz, pf, sz, plane_s);
-  if (!FFDE) count_newton(a, niter);
+  {
+    double pr[NPR];
+#pragma unroll
+    for (int k = 0; k < NPR; k++) pr[k] = __ldg(pb + k * pl + z);
+    State<double> q;
+    state_of(pr, g, q);
+    double acc[4] = {0., 0., 0., 0.};
+#pragma unroll
+    for (int jj = 0; jj < 4; jj++) {
+      double row[4];
+      mhd_row<double, FFDE>(pr, jj, q, gam, row);
+      source_row(row, jj, sz, plane_s, acc);
+    }
+    dUg[RHO] = 0. + g.g * 0.;
+    dUg[B1] = dUg[B2] = dUg[B3] = dUg[RHO];
+#pragma unroll
+    for (int l = 0; l < 4; l++) dUg[UU + l] = 0. + g.g * acc[l];
+  }
+  {
+    // the RK combine of dUtoU, advance.c:273-286
+    const double cdt = c2 * dt;
+#pragma unroll
+    for (int k = 0; k < NPR; k++) U[k] = 1.0 * U[k] + 0.0 * 0.0 + cdt * (dUr[k] + dUg[k]);
+  }
+  if constexpr (FFDE) {
+    // Utoprim_ffde, then fixup1zone's Lorentz-factor limit (the floors are
+    // GRMHD-only, fixup.c:293); pflag is left as it was
+    int rc = utoprim_ffde(U, g, pfz, a.pp.gammamax);
+    if (!rc) rc = limit_gamma(a.pp.gammamax, pfz, g);
+    if (rc) report_fail(a.sc, a.phase0 + PH_UPDATE, rc, zone_order(i, j));
+#pragma unroll
+    for (int k = 0; k < NPR; k++) pf[k * pl + z] = pfz[k];
+  } else {
+    int niter;
+    const int pfl = utoprim_2d(U, g, pfz, gam, a.pp.gammafail, &niter, NEWTON_MAIN_CAP, a.fixbuf + z, pl);
+    if (pfl == NEWTON_DEFERRED || (a.pp.tryagain && pfl != 0)) {
+      defer_zone(a, z, pfl, U);
+      niter = 0;
+    } else {
+      finish_zone(a, g, z, i, j, pfz, pfl, pf, sz[(GEO_FLOOR - GEO_CONN) * plane_s],
+                  sz[(GEO_FLOOR + 1 - GEO_CONN) * plane_s]);
+    }
+    count_newton(a, niter);
+  }
 }
 
 void launch_update_mixed(int ffde, dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map,
