@@ -837,7 +837,9 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
   }
   __syncthreads();
   // whether one of the states of the warp's faces holds a velocity or field
-  // so small that quotients may leave Exact's range
+  // so small that quotients may leave Exact's range (lane 0 has no x1 face and
+  // its left slot is not written: it looks at lane 1's)
+  const double* slot0 = slot + (tx == 0);
   bool small = false;
 #pragma unroll
   for (int q = 0; q < 4; q++)
@@ -845,7 +847,7 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
     for (int k = U1; k <= B3; k++) {
       if (!(q < 2 ? does1 : does2)) continue;
       // (volatile: these values are read again where they are used)
-      const double v = *const_cast<const volatile double*>(slot + (q * NPR + k) * KS);
+      const double v = *const_cast<const volatile double*>((q == 0 ? slot0 : slot) + (q * NPR + k) * KS);
       const uint32_t t = hi_word(v) & 0x7fffffffu;
       small |= (t < Exact::word(-850)) && ((t | lo_word(v)) != 0);
     }
