@@ -82,7 +82,7 @@ struct harm_ctx {
   int flux_by;       // k_flux rows per block (flux_rows)
   bool geo_ok;
   int sparse;        // the uploaded metric is of the sparse form (SP in harm_step_impl.cuh)
-  bool in_ensemble;  // captured into an ensemble's graph, which outlives an upload
+  int ens_blocks;    // captured into an ensemble's graph (which outlives an upload): its members' k_flux blocks
   cudaGraph_t graph;
   cudaGraphExec_t gexec;
   bool have_graph;
@@ -113,7 +113,8 @@ struct harm_ctx {
     a.geo = d_geo;
     a.geo32 = d_geo32;
     a.sparse = sparse;
-    a.sparse32 = sparse && !in_ensemble;
+    a.sparse32 = sparse && !ens_blocks;
+    a.ens_blocks = ens_blocks;
     a.geo_full = reinterpret_cast<const int*>(d_geo + GEO_NPLANES * gr.plane);
     a.F1 = d_F1;
     a.F2 = d_F2;
@@ -906,6 +907,8 @@ int harm_ensemble_create(harm_ctx* const* members, int n, int per_launch, void* 
     if (!members[k] || !members[k]->geo_ok) return HARM_EINVAL;
   harm_ensemble* e = new harm_ensemble();
   e->m.assign(members, members + n);
+  int ens_blocks = 0;
+  for (const harm_ctx* c : e->m) ens_blocks += c->nblocks_flux;
   e->per_launch = per_launch;
   e->stream = (cudaStream_t)stream;
   e->own_stream = false;
@@ -939,7 +942,7 @@ int harm_ensemble_create(harm_ctx* const* members, int n, int per_launch, void* 
       cap_ok = cudaStreamWaitEvent(br[k], ev[n], 0) == cudaSuccess;
       harm_ctx tmp = *e->m[k];
       tmp.stream = br[k];
-      tmp.in_ensemble = true;
+      tmp.ens_blocks = ens_blocks;
       for (int sidx = 0; sidx < per_launch && cap_ok; sidx++) cap_ok = enqueue_step(&tmp) == HARM_OK;
       if (cap_ok) cap_ok = cudaEventRecord(ev[k], br[k]) == cudaSuccess;
       if (cap_ok) cap_ok = cudaStreamWaitEvent(e->stream, ev[k], 0) == cudaSuccess;

@@ -101,6 +101,7 @@ struct StepArgs {
   double* rec_pinv;      // adjoint recording (or null): inverted prims before the floors, 8 planes
   unsigned char* rec_fixset;  // adjoint recording (or null): neighbour set of each repaired zone
   int nblocks_flux;
+  int ens_blocks;        // k_flux blocks of all members of the ensemble this is captured for (0: a step of its own)
   int phase0;            // PH_PER_SUBSTEP * substep: the fail-key phase of this launch's substep
   int flags_here;        // k_flux forms every zone's b^2 flags and flux choice (the first substep, FP64, fluxadjust)
   DevScalars* sc;

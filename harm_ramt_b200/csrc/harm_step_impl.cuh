@@ -900,8 +900,13 @@ inline void flux_launch_by(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, co
   // blocks each), each direction gets a layer of blocks of its own, and a
   // block half the work: a step of the 64^2 torus 71.3 -> 65.3 us, 128^2 79.6
   // -> 75.2, 245 x 131 90.9 -> 86.2 (the next size up fills the SMs anyway).
+  // An ensemble's members fill the SMs together, and the layers only repeat
+  // the tile's copy, where their blocks no longer all fit at once (a step of
+  // 2 tori of 64^2 with layers 71.8 us, without 78.4; 4 of 96^2 92.6, 93.5; 3
+  // of 128^2 102.9, 103.7; 4 of 128^2 123.0, 119.8; 16 of 128^2 with the switch
+  // 396, 360; 16 uneven ones 919, 884).
   constexpr bool small = fp64 && BY == FLUX_BY_SMALL;
-  if (small && g.x * g.y <= 2 * 148) g.z = 2;
+  if (small && g.x * g.y <= 2 * 148 && a.ens_blocks <= 4 * 148) g.z = 2;
   if constexpr (small) kern = (g.z == 2) ? k_flux_fp64<PARA, FFDE, BY, true, SP> : k_flux_fp64<PARA, FFDE, BY, false, SP>;
   else if constexpr (fp64) kern = k_flux_fp64<PARA, FFDE, BY, false, SP>;
   else kern = k_flux<T, PARA, FFDE, BY, SP>;

@@ -58,3 +58,20 @@ def test_autotune_sets_a_candidate(harm):
     assert up in autotune.UPDATE_CANDIDATES and sm in autotune.SMALL_CANDIDATES
     assert h.get_tiles() == (up, sm) and len(table) == len(autotune.UPDATE_CANDIDATES) + len(autotune.SMALL_CANDIDATES)
     assert all(v > 0 for v in table.values())
+
+
+def test_many_small_members_match_members_stepped_alone(harm):
+    """Members whose face kernels no longer fit the device at once (each runs
+    them in one layer of blocks, alone in one per direction)."""
+    from harm_ramt_b200 import ensemble
+    specs = [dict(n1=128, n2=128, a=0.1 * k, beta=50.0, torus_rmax=12.0) for k in range(4)]
+    a, b = ([h for h, _ in ensemble.build(harm, specs, lim=4, fluxmethod=1, fluxadjust=3)] for _ in range(2))
+    e = harm.Ensemble(a)
+    e.step(10)
+    st = e.sync()
+    for k, (x, y) in enumerate(zip(a, b)):
+        y.step_ch(10)
+        sy = y.sync()
+        assert all(np.array_equal(u, v) for u, v in zip(x.get_prims() + x.get_fluxes(), y.get_prims() + y.get_fluxes())), k
+        assert (st[k]["t"], st[k]["dt"]) == (sy["t"], sy["dt"])
+    e.close()
