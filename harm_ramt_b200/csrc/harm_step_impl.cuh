@@ -669,7 +669,7 @@ static __device__ __noinline__ int flux_flags_x(const StepArgs& a, const double*
 // 256 dipole; with PARA's states formed by block_states 270 -> 246 at 512^2;
 // all with the same bits.
 template <typename T, bool PARA, bool FFDE, int BY, bool SP>
-__global__ void __launch_bounds__(32 * BY, (BY == FLUX_BY_SMALL) ? 5 : 1)
+__global__ void __launch_bounds__(32 * BY, 5)
     k_flux(const __grid_constant__ StepArgs a, const __grid_constant__ CUtensorMap prim_map)
 {
   extern __shared__ __align__(128) double tile[];
@@ -920,8 +920,14 @@ inline void flux_launch_by(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, co
 template <typename T, bool PARA, bool FFDE, bool SP>
 inline void flux_rows_launch(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map)
 {
-  if (b.y == FLUX_BY_LARGE) flux_launch_by<T, PARA, FFDE, FLUX_BY_LARGE, SP>(g, b, s, a, map);
-  else flux_launch_by<T, PARA, FFDE, FLUX_BY_SMALL, SP>(g, b, s, a, map);
+  // (the FP32 faces' blocks have 4 rows on any grid, flux_rows)
+  if constexpr (sizeof(T) == 8) {
+    if (b.y == FLUX_BY_LARGE) {
+      flux_launch_by<T, PARA, FFDE, FLUX_BY_LARGE, SP>(g, b, s, a, map);
+      return;
+    }
+  }
+  flux_launch_by<T, PARA, FFDE, FLUX_BY_SMALL, SP>(g, b, s, a, map);
 }
 
 // flux_ct corner EMF, step_ch.c:1214-1234, over i in [0,N1], j in [0,N2].
