@@ -1049,8 +1049,8 @@ void launch_update(int mixed, int ffde, dim3 g, dim3 b, cudaStream_t s, const St
   } else {
     auto kern = ffde ? (a.sparse ? k_update<true, true> : k_update<true, false>)
                      : (a.sparse ? k_update<false, true> : k_update<false, false>);
-    static bool attr[4] = {false, false, false, false};
-    update_launch(kern, attr[2 * (ffde != 0) + (a.sparse != 0)], g, b, s, a, map, pi, pb, pf, c2);
+    static SmemLimit limit[4];
+    update_launch(kern, limit[2 * (ffde != 0) + (a.sparse != 0)], g, b, s, a, map, pi, pb, pf, c2);
   }
   if (!ffde) {
     if (a.pp.tryagain) k_update_tail_chain<<<148, 32 * TAIL_CHAIN, 0, s>>>(a, pi, pf);

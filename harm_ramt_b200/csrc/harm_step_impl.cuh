@@ -7,6 +7,7 @@
 #include <float.h>
 #include "harm_exact.cuh"
 #include "harm_kernels.cuh"
+#include "harm_smem.h"
 #include "harm_tma.cuh"
 
 namespace harm {
@@ -886,8 +887,7 @@ __global__ void __launch_bounds__(32 * BY, 512 / (32 * BY))
   flux_block_dt(a, dt1, dt2, sh);
 }
 
-// the k_flux instance of the block's row count (b.y) and the metric's form;
-// its dynamic shared memory limit raised once to its size
+// the k_flux instance of the block's row count (b.y) and the metric's form
 template <typename T, bool PARA, bool FFDE, int BY, bool SP>
 inline void flux_launch_by(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map)
 {
@@ -910,11 +910,8 @@ inline void flux_launch_by(dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, co
   if constexpr (small) kern = (g.z == 2) ? k_flux_fp64<PARA, FFDE, BY, true, SP> : k_flux_fp64<PARA, FFDE, BY, false, SP>;
   else if constexpr (fp64) kern = k_flux_fp64<PARA, FFDE, BY, false, SP>;
   else kern = k_flux<T, PARA, FFDE, BY, SP>;
-  static bool attr[2] = {false, false};
-  if (!attr[g.z - 1]) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    attr[g.z - 1] = true;
-  }
+  static SmemLimit limit[2];
+  limit[g.z - 1].raise((const void*)kern, sm);
   kern<<<g, b, sm, s>>>(a, map);
 }
 template <typename T, bool PARA, bool FFDE, bool SP>
@@ -1511,23 +1508,14 @@ __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepA
   }
 }
 
-// launches a k_update instance (its dynamic shared memory limit raised once
-// to the largest box of the tile shapes harm_set_tiles accepts: 42 planes x
-// at most 128 threads)
-inline void update_launch(void (*kern)(StepArgs, CUtensorMap, const double*, const double*, double*, double), bool& attr,
-                          dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map, const double* pi,
-                          const double* pb, double* pf, double c2)
+// launches a k_update instance (its dynamic shared memory limit raised to the
+// largest box of the tile shapes harm_set_tiles accepts, an even width and at
+// most 128 threads: 64 rows of 2)
+inline void update_launch(void (*kern)(StepArgs, CUtensorMap, const double*, const double*, double*, double),
+                          SmemLimit& limit, dim3 g, dim3 b, cudaStream_t s, const StepArgs& a, const CUtensorMap& map,
+                          const double* pi, const double* pb, double* pf, double c2)
 {
-  if (!attr) {
-    size_t mx = 0;
-    for (int by = 1; by <= 128; by++) {
-      const int bx = 128 / by;
-      const size_t v = upd_smem_bytes(bx + (bx & 1), by);
-      if (v > mx) mx = v;
-    }
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx);
-    attr = true;
-  }
+  limit.raise((const void*)kern, upd_smem_bytes(2, 64));
   kern<<<g, b, upd_smem_bytes(b.x, b.y), s>>>(a, map, pi, pb, pf, c2);
 }
 

@@ -130,8 +130,8 @@ void launch_update_mixed(int ffde, dim3 g, dim3 b, cudaStream_t s, const StepArg
                          const double* pi, const double* pb, double* pf, double c2)
 {
   auto kern = ffde ? k_update_mixed<true> : k_update_mixed<false>;
-  static bool attr[2] = {false, false};
-  update_launch(kern, attr[ffde != 0], g, b, s, a, map, pi, pb, pf, c2);
+  static SmemLimit limit[2];
+  update_launch(kern, limit[ffde != 0], g, b, s, a, map, pi, pb, pf, c2);
 }
 
 }  // namespace harm
