@@ -193,7 +193,10 @@ static bool encode_geo_map(CUtensorMap* map, const double* geo, const Grid& gr, 
                            UPD_STAGED);
 }
 
-// kernel classes of one step, in launch order (for per-kernel timing)
+// kernel classes of one step, in launch order (for per-kernel timing; their
+// numbers are harm_profile_step's interface, so the first one keeps its place
+// although its kernel is gone: the b^2 flags are formed in k_update and k_emf,
+// or in k_flux)
 enum { KC_BSQ = 0, KC_FLUX, KC_EMF, KC_UPDATE, KC_BOUND, KC_POLE, KC_GCHECK, KC_CHECKSOL, KC_CHECKSERIAL, KC_FIXC,
        KC_FIXA, KC_DT, KC_HORIZON, KC_FARADAY, KC_CURRENT, KC_COUNT };
 // (KC_FIXA: k_fixup_apply on the adjoint's recording path, k_bound_fix --

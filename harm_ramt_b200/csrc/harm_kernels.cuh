@@ -191,9 +191,10 @@ __device__ __forceinline__ double gdet_at(const StepArgs& a, int loc, long long 
 // rows (four 128-thread blocks per SM) on smaller grids.  Measured on the
 // developed 512^2 torus (step time, three runs each): 8 rows 0.5373-0.5405
 // ms, 16 rows (one 512-thread block per SM) 0.5427-0.5463, 15 rows (one
-// block per SM, 4.0 waves) 0.5770-0.5799.  The FP32 faces of the mixed form
-// fit 128 registers without spilling and run best as 4-row blocks at four
-// per SM on any grid.
+// block per SM, 4.0 waves) 0.5770-0.5799 (of the faces with
+// branches; of the present ones 4 rows take 94 us a launch instead of 86 at
+// 512^2 and 262 instead of 221 at 896^2).  The FP32 faces of the mixed form
+// take 96 registers and run best as 4-row blocks, five per SM, on any grid.
 #ifndef HARM_FLUX_BY_LARGE
 #define HARM_FLUX_BY_LARGE 8
 #endif

@@ -202,7 +202,8 @@ __device__ __forceinline__ void face_flux(const StepArgs& a, int i, int j, int d
 // space), found when the geometry is uploaded.  Its sums leave out the terms
 // that are a finite value times an exact zero, and those planes are not read:
 // k_flux of the 512^2 torus 87 -> 79.5 us, 1024^2 292 -> 268, the 512 x 256
-// dipole 40 -> 34.5; k_update 51 and 58 -> 49 and 53, 1024^2 178 -> 160.
+// dipole 40 -> 34.5; k_update 51 and 58 -> 49 and 53, 1024^2 178 -> 160 (the
+// faces have since gained checks: 1024^2 270).
 constexpr int SP_COV = (1 << 2) | (1 << 5) | (1 << 8), SP_CON = SP_COV | (1 << 3);
 template <bool SP>
 __device__ __forceinline__ void lower_cov(const double* v, const double* c, double* w)
@@ -665,10 +666,10 @@ static __device__ __noinline__ int flux_flags_x(const StepArgs& a, const double*
 // FP32 faces (mixed form): both directions through one copy of the face
 // code, dir a run-time value (the direction-dependent reads are selects),
 // which halves the kernel's instruction footprint.  96 registers a thread:
-// five 4-row blocks per SM.  With the sparse metric's planes and products left
-// out a mixed step takes 276 -> 270 us at 512^2 and 94.4 -> 88.0 on the 512 x
-// 256 dipole; with PARA's states formed by block_states 270 -> 246 at 512^2;
-// all with the same bits.
+// five 4-row blocks per SM.  Leaving out the sparse metric's planes and
+// products takes 6 us off a mixed step at 512^2 and 6.4 off the 512 x 256
+// dipole's, forming PARA's states by block_states 24 at 512^2; all with the
+// same bits.  49 us a launch at 512^2 PARA with the switch, 23 on the dipole.
 template <typename T, bool PARA, bool FFDE, int BY, bool SP>
 __global__ void __launch_bounds__(32 * BY, 5)
     k_flux(const __grid_constant__ StepArgs a, const __grid_constant__ CUtensorMap prim_map)
@@ -727,7 +728,7 @@ __global__ void __launch_bounds__(32 * BY, 5)
     } else {
       // MC's slopes are cheap: each thread forms its own zone's, and the left
       // state comes by shuffle or through shared memory (the mixed 512 x 256
-      // dipole 88.2 us a step, with block_states 90.9)
+      // dipole 88.2 us a step then, with block_states 90.9)
       const int st = (dir == 1) ? 1 : FLUX_TILE_W;
       T R[NPR];
 #pragma unroll
@@ -1390,8 +1391,10 @@ __device__ __forceinline__ void count_newton(const StepArgs& a, int niter)
 // between (harm_exact.cuh), at 168 registers (12 warps per SM; at 128 the
 // loads come in small batches and 172 B of registers spill: 66.6 against 61.5
 // us with the tail at 512^2).  A zone whose values leave the exact range goes
-// to update_general.  512^2 developed flow: 86 -> 50 us (first substep) and
-// 58 us (second), 3.9 TB/s; 1024^2 with the tail 300 -> 178 us.
+// to update_general.  512^2 developed flow, the kernel for any metric: 86 -> 50
+// us (first substep) and 58 us (second), 3.9 TB/s; 1024^2 with the tail 300 ->
+// 178 us.  The torus's and the star's metrics take the SP kernel: 49 and 53
+// us, 1024^2 with the tail 160.
 template <bool FFDE, bool SP>
 __global__ void __launch_bounds__(128, 3) k_update(const __grid_constant__ StepArgs a,
                                                    const __grid_constant__ CUtensorMap geo_map,
