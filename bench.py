@@ -862,8 +862,8 @@ KERNEL_BYTES_SWITCH = {"k_flux": KERNEL_BYTES["k_flux"] + (8 * 14 + 2 + 1) / 2}
 # captures of both substeps' launches at 512^2 in the developed flow
 # (sm__inst_executed_pipe_fp64.sum x 32 / zones; profiles/k_flux_*, k_update_*;
 # the first substep's k_flux also forms the flags: 2275 and 2065; k_update
-# 1320 and 1454)
-FP64_INSTR_PER_ZONE = {"k_flux": 2170, "k_update": 1387}
+# 1328 and 1462)
+FP64_INSTR_PER_ZONE = {"k_flux": 2170, "k_update": 1395}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch from the same
 # captures (mean of both substeps), scaled by zone count
 TRAFFIC_512 = {"k_flux": 92.8e6, "k_update": 186.4e6}
